@@ -322,6 +322,255 @@ static int pick_split(const RecurrenceArgs& a, int num_seqs, cudaStream_t stream
     return SHISO_ERR_SHAPE;
 }
 
+// ---- long portions, key size 64 ------------------------------------------------------------
+// The kernel above lets the threads that walk the state also convert, exponentiate or rotate what
+// a batch brings; with one warp to a scheduler nothing hides either, and a token costs some 1,500
+// cycles (1.58 ms for 2,000 tokens of 32 heads of 64 x 64).  Here a CTA holds 16 value columns of
+// a head in four warps that do nothing but walk, and four more warps stage the next batch of 16
+// tokens into the other of two buffers meanwhile: one barrier a batch.  What bounds it then is the
+// walk's own arithmetic: a lane has 8 rows of one column as four pairs for the packed multiply-adds
+// (fma.rn.f32x2), 20 of them a token with a channel decay and 12 with a head's, beside six (four)
+// 16-byte reads of shared memory.  Rows 8p..8p+3 of all parts p lie side by side in a staged vector,
+// then rows 8p+4..8p+7, so that the eight parts of a read take one pass over the banks.  The eight
+// partial sums of a column meet over 16 tokens at once: every exchange halves the tokens a lane
+// keeps, 14 shuffles instead of 48.
+constexpr int WALK_DIM = 64, WALK_COLS = 16, WALK_BATCH = 16;
+constexpr int WALK_THREADS = 256;  // four warps walk, four stage
+
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair_of(float x, float y) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float pair_sum(f32x2 v) {
+    float x, y;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v));
+    return x + y;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
+// four neighbouring activations in one load, kept as they are until they are staged
+template <typename AT> struct Four;
+template <> struct Four<float> {
+    float4 v;
+    __device__ __forceinline__ void load(const float* p) { v = *reinterpret_cast<const float4*>(p); }
+    __device__ __forceinline__ void get(float (&f)[4]) const { f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w; }
+};
+template <> struct Four<__nv_bfloat16> {
+    uint2 v;
+    __device__ __forceinline__ void load(const __nv_bfloat16* p) { v = *reinterpret_cast<const uint2*>(p); }
+    __device__ __forceinline__ void get(float (&f)[4]) const {
+        f[0] = __uint_as_float(v.x << 16); f[1] = __uint_as_float(v.x & 0xffff0000u);
+        f[2] = __uint_as_float(v.y << 16); f[3] = __uint_as_float(v.y & 0xffff0000u);
+    }
+};
+
+template <typename AT, bool CHANNEL>
+__global__ void __launch_bounds__(WALK_THREADS) decay_walk_kernel(const RecurrenceArgs a) {
+    struct Buffer {
+        float q[WALK_BATCH][WALK_DIM], k[WALK_BATCH][WALK_DIM], loss[CHANNEL ? WALK_BATCH : 1][WALK_DIM];  // loss: -(1 - w)
+        float v[WALK_BATCH][WALK_COLS];
+    };
+    __shared__ __align__(16) Buffer buffers[2];
+    const int head = blockIdx.x, seq = blockIdx.y, col0 = blockIdx.z * WALK_COLS;
+    const int tid = threadIdx.x;
+    const int vdim = a.vdim;
+    pdl_wait();
+    const int first = a.q_start[seq], last = a.q_start[seq + 1];
+    if (last <= first) return;
+    const int batches = (last - first + WALK_BATCH - 1) / WALK_BATCH;
+
+    if (tid >= 128) {
+        // ---- staging: chunk e of a batch is channels 4 (e % 16) .. + 3 of token e / 16
+        constexpr int CHUNKS = WALK_BATCH * WALK_DIM / 4 / 128;
+        const int s = tid - 128;
+        const int c = (s % 16) * 4, token0 = s / 16;
+        const int place = (c % 8 < 4) ? (c / 8) * 4 : 32 + (c / 8) * 4;  // of row c in a staged vector
+        const int half = a.rotary_dim / 2;
+        const bool turns = !CHANNEL && c < a.rotary_dim;
+        const int other = turns ? (c < half ? c + half : c - half) : c;
+        float constant[4];  // the channels' decay bias, or their rotation frequency
+#pragma unroll
+        for (int x = 0; x < 4; ++x)
+            constant[x] = CHANNEL ? a.decay_bias[head * WALK_DIM + c + x] : (turns ? a.inv_freq[(c < half ? c : c - half) + x] : 0.0f);
+        const AT* q = (const AT*)a.q + (size_t)head * WALK_DIM;
+        const AT* k = (const AT*)a.k + (size_t)head * WALK_DIM;
+        const AT* v = (const AT*)a.v + (size_t)head * vdim + col0 + (s % 4) * 4;
+        Four<AT> rq[CHUNKS], rk[CHUNKS], rq_other[CHUNKS], rk_other[CHUNKS], rv;
+        float4 logit[CHUNKS];
+        int position[CHUNKS];
+        // (a token index beyond the sequence's last is the last: every load has a valid address)
+        auto fetch = [&](int b) {
+            const int t0 = first + b * WALK_BATCH;
+#pragma unroll
+            for (int l = 0; l < CHUNKS; ++l) {
+                const int t = min(t0 + token0 + l * 8, last - 1);
+                rq[l].load(q + (size_t)t * a.q_ld + c);
+                rk[l].load(k + (size_t)t * a.k_ld + c);
+                if (CHANNEL) {
+                    logit[l] = *reinterpret_cast<const float4*>(a.decay_logits + (size_t)t * a.logits_ld + head * WALK_DIM + c);
+                } else {
+                    rq_other[l].load(q + (size_t)t * a.q_ld + other);
+                    rk_other[l].load(k + (size_t)t * a.k_ld + other);
+                    position[l] = a.rotary_dim ? a.positions[t] : 0;
+                }
+            }
+            if (s < WALK_BATCH * 4) rv.load(v + (size_t)min(t0 + s / 4, last - 1) * a.v_ld);
+        };
+        auto stage = [&](Buffer& to) {
+#pragma unroll
+            for (int l = 0; l < CHUNKS; ++l) {
+                const int i = token0 + l * 8;
+                float fq[4], fk[4];
+                rq[l].get(fq);
+                rk[l].get(fk);
+                if (CHANNEL) {
+                    const float z[4] = {logit[l].x, logit[l].y, logit[l].z, logit[l].w};
+                    float loss[4];
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) loss[x] = expm1f(-expf(z[x] + constant[x]));
+                    *reinterpret_cast<float4*>(&to.loss[i][place]) = make_float4(loss[0], loss[1], loss[2], loss[3]);
+                } else {
+                    if (turns) {
+                        float oq[4], ok[4];
+                        rq_other[l].get(oq);
+                        rk_other[l].get(ok);
+#pragma unroll
+                        for (int x = 0; x < 4; ++x) {
+                            float sn, cs;
+                            sincosf((float)position[l] * constant[x], &sn, &cs);
+                            if (c < half) sn = -sn;
+                            fq[x] = fq[x] * cs + oq[x] * sn;
+                            fk[x] = fk[x] * cs + ok[x] * sn;
+                        }
+                    }
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) fk[x] *= a.key_scale;
+                }
+                *reinterpret_cast<float4*>(&to.q[i][place]) = make_float4(fq[0], fq[1], fq[2], fq[3]);
+                *reinterpret_cast<float4*>(&to.k[i][place]) = make_float4(fk[0], fk[1], fk[2], fk[3]);
+            }
+            if (s < WALK_BATCH * 4) {
+                float fv[4];
+                rv.get(fv);
+                *reinterpret_cast<float4*>(&to.v[s / 4][(s % 4) * 4]) = make_float4(fv[0], fv[1], fv[2], fv[3]);
+            }
+        };
+        fetch(0);
+        stage(buffers[0]);
+        if (batches > 1) fetch(1);
+        for (int b = 0; b < batches; ++b) {
+            __syncthreads();  // batch b is staged, batch b - 1 is walked
+            if (b + 1 < batches) stage(buffers[(b + 1) & 1]);
+            if (b + 2 < batches) fetch(b + 2);
+        }
+        pdl_trigger();
+        return;
+    }
+
+    // ---- the walk: lanes 8c..8c+7 share column c of the warp's four, 8 rows of the state each
+    const int part = tid & 7, column = tid >> 3;
+    const int j = col0 + column, row0 = part * 8;
+    float* state = a.state + (long long)a.slots[seq] * a.state_stride + (size_t)head * WALK_DIM * vdim;
+    f32x2 S[4], bonus[4];
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        S[p] = pair_of(state[(size_t)(row0 + 2 * p) * vdim + j], state[(size_t)(row0 + 2 * p + 1) * vdim + j]);
+        bonus[p] = CHANNEL ? pair_of(a.bonus[head * WALK_DIM + row0 + 2 * p], a.bonus[head * WALK_DIM + row0 + 2 * p + 1]) : 0ull;
+    }
+    const float head_loss = CHANNEL ? 0.0f : -a.head_loss[head];
+    const f32x2 loss_all = pair_of(head_loss, head_loss);
+    float* raw = a.raw + (size_t)head * vdim + j;
+    auto token = [&](const Buffer& from, int i) {
+        const float vj = from.v[i][column];
+        const f32x2 vv = pair_of(vj, vj);
+        f32x2 o[2] = {0ull, 0ull};
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const ulonglong2 q2 = *reinterpret_cast<const ulonglong2*>(&from.q[i][h * 32 + part * 4]);
+            const ulonglong2 k2 = *reinterpret_cast<const ulonglong2*>(&from.k[i][h * 32 + part * 4]);
+            ulonglong2 w2 = make_ulonglong2(loss_all, loss_all);
+            if (CHANNEL) w2 = *reinterpret_cast<const ulonglong2*>(&from.loss[i][h * 32 + part * 4]);
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                f32x2& s2 = S[2 * h + e];
+                const f32x2 qe = e ? q2.y : q2.x, ke = e ? k2.y : k2.x, we = e ? w2.y : w2.x;
+                if (CHANNEL) o[e] = fma2(qe, fma2(bonus[2 * h + e], mul2(ke, vv), s2), o[e]);
+                s2 = fma2(ke, vv, fma2(we, s2, s2));
+                if (!CHANNEL) o[e] = fma2(qe, s2, o[e]);
+            }
+        }
+        return pair_sum(o[0]) + pair_sum(o[1]);
+    };
+    for (int b = 0; b < batches; ++b) {
+        __syncthreads();  // batch b is staged
+        const Buffer& from = buffers[b & 1];
+        const int t0 = first + b * WALK_BATCH, n = min(WALK_BATCH, last - t0);
+        float o[WALK_BATCH];
+        if (n == WALK_BATCH) {
+#pragma unroll
+            for (int i = 0; i < WALK_BATCH; ++i) o[i] = token(from, i);
+        } else {
+#pragma unroll
+            for (int i = 0; i < WALK_BATCH; ++i) {
+                o[i] = 0.0f;
+                if (i < n) o[i] = token(from, i);
+            }
+        }
+#pragma unroll
+        for (int bit = 1, kept = WALK_BATCH / 2; bit < 8; bit *= 2, kept /= 2) {
+            const bool upper = part & bit;
+#pragma unroll
+            for (int i = 0; i < WALK_BATCH / 2; ++i) {
+                if (i < kept) {
+                    const float mine = upper ? o[2 * i + 1] : o[2 * i], theirs = upper ? o[2 * i] : o[2 * i + 1];
+                    o[i] = mine + __shfl_xor_sync(0xffffffffu, theirs, bit);
+                }
+            }
+        }
+        // now o[i] is the sum of token 8 i + part
+#pragma unroll
+        for (int i = 0; i < WALK_BATCH / 8; ++i)
+            if (8 * i + part < n) raw[(size_t)(t0 + 8 * i + part) * a.heads * vdim] = o[i];
+    }
+    pdl_trigger();
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+        float x, y;
+        asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(S[p]));
+        state[(size_t)(row0 + 2 * p) * vdim + j] = x;
+        state[(size_t)(row0 + 2 * p + 1) * vdim + j] = y;
+    }
+}
+
+// What the walk reads four values at a time has to lie on their boundary.
+static bool walk_takes(const RecurrenceArgs& a, int act_dtype) {
+    const uintptr_t four = act_dtype == SHISO_F32 ? 16 : 8;
+    auto aligned = [](const void* p, uintptr_t to) { return (uintptr_t)p % to == 0; };
+    if (!a.raw || a.dim != WALK_DIM || a.vdim % WALK_COLS || a.col_parts != a.vdim / WALK_COLS) return false;
+    if (!aligned(a.q, four) || !aligned(a.k, four) || !aligned(a.v, four) || a.q_ld % 4 || a.k_ld % 4 || a.v_ld % 4) return false;
+    if (a.decay_logits) return aligned(a.decay_logits, 16) && a.logits_ld % 4 == 0;
+    return a.rotary_dim % 8 == 0;  // four channels turn together
+}
+
+template <typename AT>
+static int launch_walk(const RecurrenceArgs& a, int num_seqs, cudaStream_t stream) {
+    const dim3 grid(a.heads, num_seqs, a.col_parts);
+    if (a.decay_logits) launch_kernel(decay_walk_kernel<AT, true>, grid, WALK_THREADS, 0, stream, a);
+    else launch_kernel(decay_walk_kernel<AT, false>, grid, WALK_THREADS, 0, stream, a);
+    return launch_status();
+}
+
 // Unit RMS over a head's value channels, times weight, silu(gate) and a constant: what follows the
 // recurrence when its outputs were left unnormalised.  A warp per (row, head).
 template <typename AT>
@@ -358,6 +607,66 @@ __global__ void unit_rms_gate_kernel(const float* __restrict__ raw, const AT* __
     }
 }
 
+// The same with a quarter of the lanes to a row of a head and 16-byte accesses: LANES = vdim / 4.
+// (2,048 rows of 32 heads of 64: 24 us with a lane's values 128 bytes apart.)
+template <typename AT, int LANES>
+__global__ void unit_rms_gate_vec_kernel(const float* __restrict__ raw, const AT* __restrict__ gate, long long gate_ld,
+                                         const float* __restrict__ out_weight, AT* __restrict__ out, long long out_ld, int tokens,
+                                         int heads, float eps, float out_scale) {
+    pdl_begin();
+    constexpr int VDIM = 4 * LANES;
+    const int sub = threadIdx.x % LANES;
+    const long long item = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / LANES;
+    const bool on = item < (long long)tokens * heads;
+    const int t = on ? (int)(item / heads) : 0, head = on ? (int)(item % heads) : 0;
+    const size_t at = (size_t)head * VDIM + sub * 4;
+    const float4 o4 = *reinterpret_cast<const float4*>(raw + (size_t)t * heads * VDIM + at);
+    Four<AT> g4;
+    if (gate) g4.load(gate + (size_t)t * gate_ld + at);
+    float o[4] = {o4.x, o4.y, o4.z, o4.w};
+    float squares = (o[0] * o[0] + o[1] * o[1]) + (o[2] * o[2] + o[3] * o[3]);
+#pragma unroll
+    for (int off = 1; off < LANES; off *= 2) squares += __shfl_xor_sync(0xffffffffu, squares, off);
+    const float unit = rsqrtf(squares / (float)VDIM + eps);
+    float g[4];
+    if (gate) g4.get(g);
+    if (!on) return;
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+        o[x] *= unit;
+        if (out_weight) o[x] *= out_weight[at + x];
+        if (gate) o[x] *= g[x] / (1.0f + expf(-g[x]));
+        o[x] *= out_scale;
+    }
+    AT* to = out + (size_t)t * out_ld + at;
+    if constexpr (sizeof(AT) == 4) {
+        *reinterpret_cast<float4*>(to) = make_float4(o[0], o[1], o[2], o[3]);
+    } else {
+        __nv_bfloat162 lo = __floats2bfloat162_rn(o[0], o[1]), hi = __floats2bfloat162_rn(o[2], o[3]);
+        *reinterpret_cast<uint2*>(to) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+    }
+}
+
+template <typename AT>
+static int launch_unit_rms_gate(const RecurrenceArgs& a, int tokens, cudaStream_t stream) {
+    const float* raw = a.raw;
+    const AT* gate = (const AT*)a.gate;
+    AT* out = (AT*)a.out;
+    const long long items = (long long)tokens * a.heads;
+    const uintptr_t four = 4 * sizeof(AT);
+    const bool wide = (uintptr_t)gate % four == 0 && (uintptr_t)out % four == 0 && a.gate_ld % 4 == 0 && a.out_ld % 4 == 0;
+    if (wide && a.vdim == 64)
+        launch_kernel(unit_rms_gate_vec_kernel<AT, 16>, ceil_div_u(items, 16), 256, 0, stream, raw, gate, a.gate_ld, a.out_weight, out,
+                      a.out_ld, tokens, a.heads, a.eps, a.out_scale);
+    else if (wide && a.vdim == 128)
+        launch_kernel(unit_rms_gate_vec_kernel<AT, 32>, ceil_div_u(items, 8), 256, 0, stream, raw, gate, a.gate_ld, a.out_weight, out,
+                      a.out_ld, tokens, a.heads, a.eps, a.out_scale);
+    else
+        launch_kernel(unit_rms_gate_kernel<AT>, ceil_div_u(items, 8), 256, 0, stream, raw, gate, a.gate_ld, a.out_weight, out, a.out_ld,
+                      tokens, a.heads, a.vdim, a.eps, a.out_scale);
+    return launch_status();
+}
+
 SHISO_API int shiso_decay_recurrence(const void* q, const void* k, const void* v, const void* gate, long long q_ld, long long k_ld,
                                      long long v_ld, long long gate_ld, void* out, long long out_ld, int act_dtype, float* state,
                                      long long state_stride, const int* q_start, const int* slots, const int* positions,
@@ -383,17 +692,12 @@ SHISO_API int shiso_decay_recurrence(const void* q, const void* k, const void* v
     a.raw = raw; a.col_parts = raw ? col_parts : 1;
     if (a.col_parts < 1 || vdim % a.col_parts || !shiso_decay_recurrence_supported(dim, vdim / a.col_parts)) return SHISO_ERR_SHAPE;
     int status;
-    if (act_dtype == SHISO_F32) status = channel ? pick_split<float, true>(a, num_seqs, stream) : pick_split<float, false>(a, num_seqs, stream);
+    if (walk_takes(a, act_dtype) && (act_dtype == SHISO_F32 || act_dtype == SHISO_BF16))
+        status = act_dtype == SHISO_F32 ? launch_walk<float>(a, num_seqs, stream) : launch_walk<__nv_bfloat16>(a, num_seqs, stream);
+    else if (act_dtype == SHISO_F32) status = channel ? pick_split<float, true>(a, num_seqs, stream) : pick_split<float, false>(a, num_seqs, stream);
     else if (act_dtype == SHISO_BF16)
         status = channel ? pick_split<__nv_bfloat16, true>(a, num_seqs, stream) : pick_split<__nv_bfloat16, false>(a, num_seqs, stream);
     else return SHISO_ERR_DTYPE;
     if (status != SHISO_OK || !raw) return status;
-    const unsigned blocks = ceil_div_u((long long)tokens * heads, 8);
-    if (act_dtype == SHISO_F32)
-        launch_kernel(unit_rms_gate_kernel<float>, blocks, 256, 0, stream, (const float*)raw, (const float*)gate, gate_ld, out_weight,
-                      (float*)out, out_ld, tokens, heads, vdim, eps, out_scale);
-    else
-        launch_kernel(unit_rms_gate_kernel<__nv_bfloat16>, blocks, 256, 0, stream, (const float*)raw, (const __nv_bfloat16*)gate, gate_ld,
-                      out_weight, (__nv_bfloat16*)out, out_ld, tokens, heads, vdim, eps, out_scale);
-    return launch_status();
+    return act_dtype == SHISO_F32 ? launch_unit_rms_gate<float>(a, tokens, stream) : launch_unit_rms_gate<__nv_bfloat16>(a, tokens, stream);
 }

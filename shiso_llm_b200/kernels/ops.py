@@ -1203,6 +1203,9 @@ def decay_recurrence(q, k, v, out, state, step, heads, dim, vdim, eps, *, decay_
     # and gate then follow in a row kernel.  The split depends on the step's shape only.
     col_parts, raw = 1, None
     if not getattr(step, "all_decode", False) and getattr(step, "max_q_len", tokens) >= RECURRENCE_SPLIT_MIN_PORTION:
+        if dim == 64 and vdim % 16 == 0:
+            # (the kernel for long portions walks 16 columns a CTA; 1.58 ms -> WALKMS for 2,000 tokens of 32 heads)
+            col_parts = vdim // 16
         while (col_parts < 8 and heads * step.num_seqs * col_parts < _sm_count() and vdim % (2 * col_parts) == 0
                and vdim // (2 * col_parts) >= 8 and recurrence_supported(dim, vdim // (2 * col_parts))):
             col_parts *= 2
