@@ -442,6 +442,13 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype, bias: Optio
         )
         _done(status, "linear (tcgen05)", shape=(tokens, n, k))
         return out
+    if x.dtype == w.dtype == out_dtype == torch.float32:
+        groups = lib.shiso_gemm_float_groups(_ptr(x), _ptr(w), _ptr(out), tokens, n, k)
+        if groups >= 0:
+            partial = torch.empty((groups, tokens, n), dtype=torch.float32, device=x.device) if groups else None
+            status = lib.shiso_gemm_float(_ptr(x), _ptr(w), _ptr(bias), _ptr(out), _ptr(partial), tokens, n, k, _stream())
+            _done(status, "linear (float)", 2 if groups else 1, shape=(tokens, n, k))
+            return out
     status = lib.shiso_gemm_simple(
         _ptr(x), _code(x), _ptr(w), _code(w), _ptr(bias), _ptr(out), _code(out), tokens, n, k, _stream()
     )
@@ -1203,13 +1210,13 @@ def decay_recurrence(q, k, v, out, state, step, heads, dim, vdim, eps, *, decay_
     # and gate then follow in a row kernel.  The split depends on the step's shape only.
     col_parts, raw = 1, None
     if not getattr(step, "all_decode", False) and getattr(step, "max_q_len", tokens) >= RECURRENCE_SPLIT_MIN_PORTION:
-        if dim == 64 and vdim % 16 == 0:
-            # (the kernel for long portions walks 16 columns a CTA; 1.58 ms -> WALKMS for 2,000 tokens of 32 heads)
+        walks = dim == 64 and vdim % 16 == 0  # the kernel that walks 16 columns a CTA, however many heads and sequences there are
+        if walks:
             col_parts = vdim // 16
-        while (col_parts < 8 and heads * step.num_seqs * col_parts < _sm_count() and vdim % (2 * col_parts) == 0
+        while (not walks and col_parts < 8 and heads * step.num_seqs * col_parts < _sm_count() and vdim % (2 * col_parts) == 0
                and vdim // (2 * col_parts) >= 8 and recurrence_supported(dim, vdim // (2 * col_parts))):
             col_parts *= 2
-        if col_parts > 1:
+        if walks or col_parts > 1:
             raw = torch.empty((tokens, heads * vdim), dtype=torch.float32, device=q.device)
     status = library().shiso_decay_recurrence(
         q.data_ptr(), k.data_ptr(), v.data_ptr(), gate.data_ptr() if gate is not None else 0, q_ld, k_ld, v_ld, gate_ld,
