@@ -1208,11 +1208,14 @@ def decay_recurrence(q, k, v, out, state, step, heads, dim, vdim, eps, *, decay_
     # Long portions: a head's value columns are shared out over several CTAs (few heads and sequences
     # would leave most SMs idle while one walks thousands of tokens); the outputs' unit RMS, weight
     # and gate then follow in a row kernel.  The split depends on the step's shape only.
-    col_parts, raw = 1, None
-    if not getattr(step, "all_decode", False) and getattr(step, "max_q_len", tokens) >= RECURRENCE_SPLIT_MIN_PORTION:
-        walks = dim == 64 and vdim % 16 == 0  # the kernel that walks 16 columns a CTA, however many heads and sequences there are
+    col_parts, raw, room = 1, None, None
+    longest = getattr(step, "max_q_len", tokens)
+    if not getattr(step, "all_decode", False) and longest >= RECURRENCE_SPLIT_MIN_PORTION:
+        walks = dim == 64 and vdim % 64 == 0  # the kernel that walks segments of a portion, 64 columns a CTA
         if walks:
-            col_parts = vdim // 16
+            col_parts = vdim // 64
+            # (a state and a decay per segment of 128 tokens: recurrence.cu, find_segment)
+            room = torch.empty(((tokens // 128 + step.num_seqs) * heads * dim * (vdim + 1),), dtype=torch.float32, device=q.device)
         while (not walks and col_parts < 8 and heads * step.num_seqs * col_parts < _sm_count() and vdim % (2 * col_parts) == 0
                and vdim // (2 * col_parts) >= 8 and recurrence_supported(dim, vdim // (2 * col_parts))):
             col_parts *= 2
@@ -1223,7 +1226,7 @@ def decay_recurrence(q, k, v, out, state, step, heads, dim, vdim, eps, *, decay_
         out.data_ptr(), out_ld, _CODES[act], state.data_ptr(), stride, _ptr(step.q_start), _ptr(step.state_slots),
         _ptr(step.positions), _ptr(decay_logits), logits_ld, _ptr(decay_bias), _ptr(bonus), _ptr(head_loss),
         _ptr(inv_freq) if rotary_dim else 0, int(rotary_dim), float(key_scale), _ptr(out_weight), float(eps), float(out_scale),
-        _ptr(raw), col_parts, tokens, step.num_seqs, heads, dim, vdim, _stream(),
+        _ptr(raw), col_parts, _ptr(room), int(longest), tokens, step.num_seqs, heads, dim, vdim, _stream(),
     )
     _done(status, "decay_recurrence" + (f" (columns over {col_parts} CTAs)" if raw is not None else ""), 2 if raw is not None else 1,
           shape=(tokens, heads, dim, vdim))

@@ -1,5 +1,5 @@
 """The walk of long portions with 64 key channels against the stand-in of the same name: portions
-that end inside, on and behind a batch of 16 tokens, single tokens beside them, both decays, both
+that end inside, on and behind a batch of 16 tokens and a segment of 128, single tokens beside them, both decays, both
 numbers of value columns, states that a step before left, and column ranges that only the general
 kernel takes."""
 
@@ -14,12 +14,12 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("kind", ["channel", "head"])
-@pytest.mark.parametrize("vdim,lead,rotary", [(64, 0, 64), (128, 4, 16), (64, 3, 64), (16, 0, 0)])
-@pytest.mark.parametrize("q_lens", [[64, 1, 80], [15, 97], [130]])
+@pytest.mark.parametrize("vdim,lead,rotary", [(64, 0, 64), (128, 4, 16), (64, 3, 64), (192, 0, 0)])
+@pytest.mark.parametrize("q_lens", [[64, 1, 80], [15, 97], [128, 129], [1, 700, 3], [256]])
 def test_walk_of_long_portions(dtype, kind, vdim, lead, rotary, q_lens):
     heads, dim, t = 3, 64, ops()
     starts = [7 * s for s in range(len(q_lens))]
-    cpu, gpu, _ = make_step(q_lens, starts, 16, 32, 3, num_slots=5)
+    cpu, gpu, _ = make_step(q_lens, starts, 16, 64, 3, num_slots=5)
     gpu.all_decode, gpu.max_q_len = False, max(q_lens)
     rows, qk, vg = sum(q_lens), heads * dim, heads * vdim
     x = rnd((rows, lead + 2 * qk + 2 * vg), dtype, 1, 0.5)
@@ -40,6 +40,6 @@ def test_walk_of_long_portions(dtype, kind, vdim, lead, rotary, q_lens):
     q, k, v, gate = parts(x.cuda())
     on_gpu = {n: (y.cuda() if torch.is_tensor(y) else y) for n, y in kw.items()}
     t.decay_recurrence(q, k, v, got[:, lead:], got_state, gpu, heads, dim, vdim, 1e-5, gate=gate, out_scale=0.5, **on_gpu)
-    # (float32 sums over at most 130 tokens of 64 channels: the bound of the general kernel's tests)
+    # (float32 sums over at most 700 tokens of 64 channels: the bound of the general kernel's tests)
     close(got[:, lead:], want, dtype, f"walk {kind} {vdim} {q_lens}", rel32=2e-5)
     close(got_state, want_state, torch.float32, f"state {kind} {vdim} {q_lens}", rel32=2e-5)
