@@ -98,6 +98,33 @@ __device__ __forceinline__ float glu_times(float g, float u, int act, float limi
     return g * r * u;
 }
 
+// ---- packed float pairs ------------------------------------------------------------------------
+// Two floats in a 64-bit register and one operation for both, each half rounded as the scalar operation
+// rounds it.  (Two packed operations may still be joined into one: a product whose own rounding counts
+// and that only an addition reads is formed with __fmul_rn.)
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pair_of(float x, float y) {
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ void halves(f32x2 v, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+
 // ---- programmatic dependent launch ---------------------------------------------------------
 // Every kernel is launched so that it may start while its predecessor in the stream is still
 // finishing.  It waits for the predecessor to complete and flush (griddepcontrol.wait) before

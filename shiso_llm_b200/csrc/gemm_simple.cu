@@ -94,24 +94,6 @@ int launch(const void* x, const void* w, const float* bias, void* y, int T, int 
 // tiles) or each group has CTAs of its own, whose sums a second kernel adds up (few tiles).
 constexpr int PN = 128, PK = 16, P_THREADS = 128;
 
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 both_of(float x) {
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
-    return r;
-}
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
-    f32x2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ void halves(f32x2 v, float& x, float& y) { asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(v)); }
-
 // TM: rows of x a thread has; a CTA has 8 TM.  ALL: the CTA walks every group of K (grid.z = 1), else
 // group blockIdx.z, whose sums go to partial[blockIdx.z][T][N].
 template <int TM, bool ALL>
@@ -195,7 +177,7 @@ gemm_float_kernel(const float* __restrict__ x, const float* __restrict__ w, cons
             const ulonglong2 b0 = *(const ulonglong2*)&ws[s][k][4 * tx], b1 = *(const ulonglong2*)&ws[s][k][PN / 2 + 4 * tx];
 #pragma unroll
             for (int i = 0; i < TM; ++i) {
-                const f32x2 ai = both_of(a[i]);
+                const f32x2 ai = pair_of(a[i], a[i]);
                 acc[i][0] = fma2(ai, b0.x, acc[i][0]);
                 acc[i][1] = fma2(ai, b0.y, acc[i][1]);
                 acc[i][2] = fma2(ai, b1.x, acc[i][2]);

@@ -1155,7 +1155,10 @@ def _rows(t, name, dtype, width=None) -> int:
     return t.stride(0)
 
 
-RECURRENCE_SPLIT_MIN_PORTION = 64  # portions from here on may share a head's value columns out over several CTAs
+# Portions from here on walk in a kernel of their own, or share a head's value columns out over several CTAs.  (One of
+# 64 rows of 32 heads of 64 x 64: 66 us in 8 CTAs a head, 16 us in the walk.)
+RECURRENCE_SPLIT_MIN_PORTION = 64
+RECURRENCE_SEGMENT = 128  # tokens of a segment of the walk (decay_walk.cu)
 
 
 def recurrence_supported(dim: int, vdim: int) -> bool:
@@ -1205,29 +1208,41 @@ def decay_recurrence(q, k, v, out, state, step, heads, dim, vdim, eps, *, decay_
         _check(out_weight, "output weight", torch.float32, 1)
         if out_weight.shape[0] != heads * vdim:
             raise KernelError(f"an output weight of {out_weight.shape[0]} for {heads} heads of {vdim}")
-    # Long portions: a head's value columns are shared out over several CTAs (few heads and sequences
-    # would leave most SMs idle while one walks thousands of tokens); the outputs' unit RMS, weight
-    # and gate then follow in a row kernel.  The split depends on the step's shape only.
-    col_parts, raw, room = 1, None, None
+    # Long portions: the state walks ahead and segments of 128 tokens follow at the same time
+    # (decay_walk.cu) where the kernel takes the operands; else a head's value columns are shared out over several
+    # CTAs (few heads and sequences would leave most SMs idle while one walks thousands of tokens).  The
+    # outputs' unit RMS, weight and gate then follow in a row kernel.  ``step.max_q_len`` chooses between them
+    # and changes no bit of a state.
+    lib = library()
+    col_parts, raw, room, walks, taken = 1, None, None, False, False
     longest = getattr(step, "max_q_len", tokens)
     if not getattr(step, "all_decode", False) and longest >= RECURRENCE_SPLIT_MIN_PORTION:
-        walks = dim == 64 and vdim % 64 == 0  # the kernel that walks segments of a portion, 64 columns a CTA
+        walks = dim == 64 and vdim % 64 == 0
         if walks:
             col_parts = vdim // 64
-            # (a state and a decay per segment of 128 tokens: recurrence.cu, find_segment)
-            room = torch.empty(((tokens // 128 + step.num_seqs) * heads * dim * (vdim + 1),), dtype=torch.float32, device=q.device)
+        taken = walks and bool(lib.shiso_decay_walk_takes(
+            _CODES[act], q.data_ptr(), k.data_ptr(), v.data_ptr(), q_ld, k_ld, v_ld, state.data_ptr(), stride,
+            _ptr(decay_logits), logits_ld, int(rotary_dim), tokens, step.num_seqs, dim, vdim,
+        ))
+        if taken:  # (decay_walk.cu, state_place)
+            room = torch.empty((2 * max(1, tokens // RECURRENCE_SEGMENT), heads, dim, vdim), dtype=torch.float32, device=q.device)
         while (not walks and col_parts < 8 and heads * step.num_seqs * col_parts < _sm_count() and vdim % (2 * col_parts) == 0
                and vdim // (2 * col_parts) >= 8 and recurrence_supported(dim, vdim // (2 * col_parts))):
             col_parts *= 2
         if walks or col_parts > 1:
             raw = torch.empty((tokens, heads * vdim), dtype=torch.float32, device=q.device)
-    status = library().shiso_decay_recurrence(
+    operands = (
         q.data_ptr(), k.data_ptr(), v.data_ptr(), gate.data_ptr() if gate is not None else 0, q_ld, k_ld, v_ld, gate_ld,
         out.data_ptr(), out_ld, _CODES[act], state.data_ptr(), stride, _ptr(step.q_start), _ptr(step.state_slots),
         _ptr(step.positions), _ptr(decay_logits), logits_ld, _ptr(decay_bias), _ptr(bonus), _ptr(head_loss),
         _ptr(inv_freq) if rotary_dim else 0, int(rotary_dim), float(key_scale), _ptr(out_weight), float(eps), float(out_scale),
-        _ptr(raw), col_parts, _ptr(room), int(longest), tokens, step.num_seqs, heads, dim, vdim, _stream(),
+        _ptr(raw),
     )
+    sizes = (tokens, step.num_seqs, heads, dim, vdim, _stream())
+    if taken:
+        status = lib.shiso_decay_walk(*operands, _ptr(room), *sizes)
+    else:
+        status = lib.shiso_decay_recurrence(*operands, col_parts, *sizes)
     _done(status, "decay_recurrence" + (f" (columns over {col_parts} CTAs)" if raw is not None else ""), 2 if raw is not None else 1,
           shape=(tokens, heads, dim, vdim))
     return out
