@@ -1214,17 +1214,14 @@ def decay_recurrence(q, k, v, out, state, step, heads, dim, vdim, eps, *, decay_
     # outputs' unit RMS, weight and gate then follow in a row kernel.  ``step.max_q_len`` chooses between them
     # and changes no bit of a state.
     lib = library()
-    col_parts, raw, room, walks, taken = 1, None, None, False, False
+    col_parts, raw, room, walks = 1, None, None, False
     longest = getattr(step, "max_q_len", tokens)
     if not getattr(step, "all_decode", False) and longest >= RECURRENCE_SPLIT_MIN_PORTION:
-        walks = dim == 64 and vdim % 64 == 0
-        if walks:
-            col_parts = vdim // 64
-        taken = walks and bool(lib.shiso_decay_walk_takes(
+        walks = bool(lib.shiso_decay_walk_takes(
             _CODES[act], q.data_ptr(), k.data_ptr(), v.data_ptr(), q_ld, k_ld, v_ld, state.data_ptr(), stride,
             _ptr(decay_logits), logits_ld, int(rotary_dim), tokens, step.num_seqs, dim, vdim,
         ))
-        if taken:  # (decay_walk.cu, state_place)
+        if walks:  # (decay_walk.cu, state_place)
             room = torch.empty((2 * max(1, tokens // RECURRENCE_SEGMENT), heads, dim, vdim), dtype=torch.float32, device=q.device)
         while (not walks and col_parts < 8 and heads * step.num_seqs * col_parts < _sm_count() and vdim % (2 * col_parts) == 0
                and vdim // (2 * col_parts) >= 8 and recurrence_supported(dim, vdim // (2 * col_parts))):
@@ -1239,7 +1236,7 @@ def decay_recurrence(q, k, v, out, state, step, heads, dim, vdim, eps, *, decay_
         _ptr(raw),
     )
     sizes = (tokens, step.num_seqs, heads, dim, vdim, _stream())
-    if taken:
+    if walks:
         status = lib.shiso_decay_walk(*operands, _ptr(room), *sizes)
     else:
         status = lib.shiso_decay_recurrence(*operands, col_parts, *sizes)

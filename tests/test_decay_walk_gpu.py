@@ -139,3 +139,22 @@ def test_a_longest_portion_that_is_wrong_costs_no_bit(kind, vdim, hint):
     right, wrong = (Portions(kind, vdim, torch.bfloat16, sum(q_lens)) for _ in range(2))
     want, got = right.step(0, q_lens, starts, slots), wrong.step(0, q_lens, starts, slots, hint=hint)
     assert torch.equal(got, want) and torch.equal(wrong.state, right.state)
+
+
+@pytest.mark.parametrize("vdim,lead,q_lens,what", [
+    (64, 3, [300], "(columns over 8 CTAs)"), (128, 3, [300], "(columns over 8 CTAs)"), (64, 0, [30, 40], "decay_recurrence"),
+])
+def test_what_the_walk_does_not_take_shares_its_columns_out(monkeypatch, vdim, lead, q_lens, what):
+    seen = launches_of(monkeypatch, lambda: Portions("head", vdim, torch.bfloat16, sum(q_lens), lead).step(
+        0, q_lens, [0] * len(q_lens), list(range(len(q_lens)))))
+    assert len(seen) == 1 and seen[0][0].endswith(what), seen
+
+
+def launches_of(monkeypatch, call):
+    """(what, launches) of every entry of the launch table that a call makes."""
+    from shiso_llm_b200.kernels import ops as table
+
+    seen, done = [], table._done
+    monkeypatch.setattr(table, "_done", lambda status, name, count=1, shape=(): (seen.append((name, count)), done(status, name, count, shape)))
+    call()
+    return seen
