@@ -1237,11 +1237,12 @@ def decay_recurrence(q, k, v, out, state, step, heads, dim, vdim, eps, *, decay_
     )
     sizes = (tokens, step.num_seqs, heads, dim, vdim, _stream())
     if walks:
-        status = lib.shiso_decay_walk(*operands, _ptr(room), *sizes)
+        status, launches = lib.shiso_decay_walk(*operands, _ptr(room), *sizes), 2 if room is None else 3
+        what = "decay_recurrence (walk)" if room is None else "decay_recurrence (walk of segments)"
     else:
-        status = lib.shiso_decay_recurrence(*operands, col_parts, *sizes)
-    _done(status, "decay_recurrence" + (f" (columns over {col_parts} CTAs)" if raw is not None else ""), 2 if raw is not None else 1,
-          shape=(tokens, heads, dim, vdim))
+        status, launches = lib.shiso_decay_recurrence(*operands, col_parts, *sizes), 1 if raw is None else 2
+        what = "decay_recurrence" + (f" (columns over {col_parts} CTAs)" if raw is not None else "")
+    _done(status, what, launches, shape=(tokens, heads, dim, vdim))
     return out
 
 

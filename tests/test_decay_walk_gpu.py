@@ -158,3 +158,13 @@ def launches_of(monkeypatch, call):
     monkeypatch.setattr(table, "_done", lambda status, name, count=1, shape=(): (seen.append((name, count)), done(status, name, count, shape)))
     call()
     return seen
+
+
+@pytest.mark.parametrize("vdim,lead,q_lens,what,launches", [
+    (64, 0, [300], "(walk of segments)", 3), (128, 0, [300, 2], "(walk of segments)", 3), (64, 3, [300], "(columns over 8 CTAs)", 2),
+    (64, 0, [30, 40], "decay_recurrence", 1),
+])
+def test_a_recurrence_counts_its_launches(monkeypatch, vdim, lead, q_lens, what, launches):
+    seen = launches_of(monkeypatch, lambda: Portions("head", vdim, torch.bfloat16, sum(q_lens), lead).step(
+        0, q_lens, [0] * len(q_lens), list(range(len(q_lens)))))
+    assert len(seen) == 1 and seen[0][0].endswith(what) and seen[0][1] == launches, seen
