@@ -129,17 +129,42 @@ def default_ops():
     return ops
 
 
+def _mixers(spec):
+    """The mixers of a layer: itself, or its branches."""
+    if "branches" in spec.params:
+        return [m for part, _ in spec.params["branches"] for m in _mixers(part)]
+    return [spec]
+
+
+def recurrence_room_bytes(plan, rows: int) -> int:
+    """What one decaying recurrence with 64 key channels takes for a step of ``rows`` rows: the states its segments of
+    128 tokens begin with (csrc/decay_walk.cu, state_place) and its outputs before their unit RMS, in float32."""
+    most = 0
+    for layer in plan.layers:
+        for spec in _mixers(layer.mixer) if layer.mixer is not None else ():
+            p = spec.params
+            if spec.kind not in ("wkv_time_mix", "retention"):
+                continue
+            heads, dim = p["num_heads"], p["head_dim"]
+            vdim = p.get("v_head_dim") or dim
+            states = 2 * (rows // 128) * heads * dim * vdim if dim == 64 else 0
+            most = max(most, 4 * (states + rows * heads * vdim))
+    return most
+
+
 def step_buffer_bytes(plan, options: EngineOptions, dtype: torch.dtype) -> int:
     """An upper bound of what one step of ``max_num_batched_tokens`` rows allocates beside
     weights and cache: the residual stream (float32, two copies), a few activations as wide as
-    the widest product's output, and the logits of one row per sequence."""
+    the widest product's output, the logits of one row per sequence, and the workspaces of the kernels that take
+    some that grows with the rows."""
     widest = max([plan.hidden_size] + [int(v) for layer in plan.layers for spec in (layer.mixer, layer.feed_forward)
                                        if spec is not None for k, v in spec.params.items()
                                        if k in ("intermediate_size", "hidden_size") and isinstance(v, int)])
     rows = options.max_num_batched_tokens
     activations = rows * (2 * plan.hidden_size * 4 + 6 * 3 * widest * dtype.itemsize)
     logits = 2 * max(options.max_num_seqs, 1) * plan.vocab_size * 4
-    return activations + logits + (256 << 20)
+    workspaces = recurrence_room_bytes(plan, rows)
+    return activations + logits + workspaces + (256 << 20)
 
 
 class Engine:

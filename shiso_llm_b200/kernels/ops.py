@@ -1221,8 +1221,8 @@ def decay_recurrence(q, k, v, out, state, step, heads, dim, vdim, eps, *, decay_
             _CODES[act], q.data_ptr(), k.data_ptr(), v.data_ptr(), q_ld, k_ld, v_ld, state.data_ptr(), stride,
             _ptr(decay_logits), logits_ld, int(rotary_dim), tokens, step.num_seqs, dim, vdim,
         ))
-        if walks:  # (decay_walk.cu, state_place)
-            room = torch.empty((2 * max(1, tokens // RECURRENCE_SEGMENT), heads, dim, vdim), dtype=torch.float32, device=q.device)
+        if walks and longest > RECURRENCE_SEGMENT and tokens > RECURRENCE_SEGMENT:  # (decay_walk.cu, state_place)
+            room = torch.empty((2 * (tokens // RECURRENCE_SEGMENT), heads, dim, vdim), dtype=torch.float32, device=q.device)
         while (not walks and col_parts < 8 and heads * step.num_seqs * col_parts < _sm_count() and vdim % (2 * col_parts) == 0
                and vdim // (2 * col_parts) >= 8 and recurrence_supported(dim, vdim // (2 * col_parts))):
             col_parts *= 2

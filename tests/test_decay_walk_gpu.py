@@ -161,7 +161,7 @@ def launches_of(monkeypatch, call):
 
 
 @pytest.mark.parametrize("vdim,lead,q_lens,what,launches", [
-    (64, 0, [300], "(walk of segments)", 3), (128, 0, [300, 2], "(walk of segments)", 3), (64, 3, [300], "(columns over 8 CTAs)", 2),
+    (64, 0, [300], "(walk of segments)", 3), (128, 0, [300, 2], "(walk of segments)", 3), (64, 0, [100, 90], "(walk)", 2), (64, 3, [300], "(columns over 8 CTAs)", 2),
     (64, 0, [30, 40], "decay_recurrence", 1),
 ])
 def test_a_recurrence_counts_its_launches(monkeypatch, vdim, lead, q_lens, what, launches):

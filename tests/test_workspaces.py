@@ -1,5 +1,15 @@
-"""Rules on the host that no GPU is needed for: which steps the walk of long portions takes."""
+"""Rules on the host that no GPU is needed for: which steps the walk of long portions takes, and that what an
+engine sets aside for a step covers the workspaces of its kernels."""
 
+import json
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from shiso_llm_b200.cli import preset_path
+from shiso_llm_b200.config import plan_from_document
+from shiso_llm_b200.engine import core
 from shiso_llm_b200.kernels.library import library
 
 AT = 0x7F0000000000  # an address on every boundary; nothing is read there
@@ -29,3 +39,17 @@ def test_which_steps_the_walk_takes():
     # what a grid has no room for stays with the general kernel
     assert walk_takes(tokens=1, seqs=65535) == 1 and walk_takes(tokens=128, seqs=65535) == 0
     assert walk_takes(tokens=128 * 65534 + 127, seqs=1) == 1 and walk_takes(tokens=128 * 65535, seqs=1) == 0
+
+
+@pytest.mark.parametrize("preset", ["filulix-1b", "filulix-350m"])
+@pytest.mark.parametrize("rows", [64, 2048, 16384])
+def test_recurrences_are_set_aside_for(preset, rows):
+    with open(preset_path(preset)) as f:
+        _, _, plan = plan_from_document(json.load(f))
+    options = SimpleNamespace(max_num_batched_tokens=rows, max_num_seqs=8)
+    # 16 heads of 64 x 128 and 32 of 64 x 64 (half as many in the smaller model): outputs in float32, two states per 128 rows
+    heads = 32 if preset == "filulix-1b" else 16
+    need = 4 * (rows * heads * 64 + 2 * (rows // 128) * heads * 64 * 64)
+    assert core.recurrence_room_bytes(plan, rows) == need
+    plain = core.step_buffer_bytes(SimpleNamespace(hidden_size=plan.hidden_size, vocab_size=plan.vocab_size, layers=[]), options, torch.bfloat16)
+    assert core.step_buffer_bytes(plan, options, torch.bfloat16) >= plain + need
