@@ -249,12 +249,14 @@ __global__ void __launch_bounds__(256) gemm_float_join_kernel(const float* __res
     for (int e = 0; e < 4 && at + e < count; ++e) y[at + e] = bias ? v[e] + bias[(at + e) % N] : v[e];
 }
 
-// The columns of K in a group: as many groups as give a single tile of tokens about a CTA for every SM,
-// of at least 128 columns each.
+// The columns of K in a group: as many groups as give a single tile of tokens about GROUP_CTAS CTAs, of at
+// least GROUP_MIN columns each.  (Both fix the order of every sum: they are no device's SM count, and N and K
+// are all that may be asked for.)
+constexpr int GROUP_CTAS = 128, GROUP_MIN = 128;
 int group_size(int N, int K) {
     const int tiles = (N + PN - 1) / PN;
-    int groups = (128 + tiles - 1) / tiles;
-    if (groups > K / 128) groups = K / 128;
+    int groups = (GROUP_CTAS + tiles - 1) / tiles;
+    if (groups > K / GROUP_MIN) groups = K / GROUP_MIN;
     if (groups < 1) groups = 1;
     return ((K + groups - 1) / groups + PK - 1) / PK * PK;
 }
@@ -266,16 +268,21 @@ bool float_takes(const void* x, const void* w, const void* y, int T, int K) {
 // Rows of a thread: 8, unless tiles of 32 rows pad T less; one row each for a handful.
 int rows_of_thread(int T) { return T <= 8 ? 1 : ((T + 31) / 32 * 32 < (T + 63) / 64 * 64 ? 4 : 8); }
 
-// One CTA walks all groups of a tile when the tiles alone give every SM two CTAs.
-bool walks_all(int T, int N, int K) {
-    const int tm = rows_of_thread(T);
-    return group_size(N, K) >= K || (long long)((T + 8 * tm - 1) / (8 * tm)) * ((N + PN - 1) / PN) >= 2 * 148;
+// One CTA walks all groups of a tile when the tiles alone give every SM two CTAs (as many as are resident with eight
+// rows a thread), or when the groups' sums would take more than ROOM floats (256 MiB: what an engine sets aside
+// for them).  Neither changes a bit.  (Groups of their own against one CTA, microseconds: 600 rows x 1,024 x 4,608 164 and
+// 329, 2,048 rows 418 and 516 with 128 MiB, 4,600 rows x 512 x 4,608 504 and 536 with 288 MiB; where the tiles suffice,
+// 2,300 rows x 1,024 x 1,024, 118 and 115.)
+constexpr long long ROOM = 1ll << 26;
+bool walks_all(int T, int N, int K, int sm_count) {
+    const int tm = rows_of_thread(T), group = group_size(N, K);
+    const long long tiles = (long long)((T + 8 * tm - 1) / (8 * tm)) * ((N + PN - 1) / PN), groups = (K + group - 1) / group;
+    return groups < 2 || tiles >= 2 * sm_count || groups * T * N > ROOM;
 }
 
 template <int TM>
-int launch_float(const float* x, const float* w, const float* bias, float* y, float* partial, int T, int N, int K, cudaStream_t stream) {
+int launch_float(const float* x, const float* w, const float* bias, float* y, float* partial, int T, int N, int K, bool all, cudaStream_t stream) {
     const int group = group_size(N, K), groups = (K + group - 1) / group;
-    const bool all = walks_all(T, N, K);
     const dim3 grid(ceil_div_u(N, PN), ceil_div_u(T, 8 * TM), all ? 1 : groups);
     if (all) {
         launch_kernel(gemm_float_kernel<TM, true>, grid, P_THREADS, 0, stream, x, w, bias, y, partial, T, N, K, group);
@@ -293,24 +300,25 @@ int launch_float(const float* x, const float* w, const float* bias, float* y, fl
 
 // Groups of K whose sums shiso_gemm_float wants room for, [groups, T, N] floats on a 16-byte boundary; 0:
 // none; -1: it does not take the product.
-SHISO_API int shiso_gemm_float_groups(const void* x, const void* w, const void* y, int T, int N, int K) {
+SHISO_API int shiso_gemm_float_groups(const void* x, const void* w, const void* y, int T, int N, int K, int sm_count) {
     if (T <= 0 || N <= 0 || K <= 0 || !float_takes(x, w, y, T, K)) return -1;
-    if (walks_all(T, N, K)) return 0;
+    if (walks_all(T, N, K, sm_count)) return 0;
     const int group = group_size(N, K);
     return (K + group - 1) / group;
 }
 
 SHISO_API int shiso_gemm_float(const void* x, const void* w, const float* bias, void* y, void* partial, int T, int N, int K,
-                               cudaStream_t stream) {
+                               int sm_count, cudaStream_t stream) {
     if (T <= 0 || N <= 0) return SHISO_OK;
     if (K <= 0) return SHISO_ERR_SHAPE;
     if (!float_takes(x, w, y, T, K)) return SHISO_ERR_ALIGN;
-    if (!walks_all(T, N, K) && (!partial || (uintptr_t)partial % 16)) return SHISO_ERR_ALIGN;
+    const bool all = walks_all(T, N, K, sm_count);
+    if (!all && (!partial || (uintptr_t)partial % 16)) return SHISO_ERR_ALIGN;
     const float *xf = (const float*)x, *wf = (const float*)w;
     switch (rows_of_thread(T)) {
-        case 1: return launch_float<1>(xf, wf, bias, (float*)y, (float*)partial, T, N, K, stream);
-        case 4: return launch_float<4>(xf, wf, bias, (float*)y, (float*)partial, T, N, K, stream);
-        default: return launch_float<8>(xf, wf, bias, (float*)y, (float*)partial, T, N, K, stream);
+        case 1: return launch_float<1>(xf, wf, bias, (float*)y, (float*)partial, T, N, K, all, stream);
+        case 4: return launch_float<4>(xf, wf, bias, (float*)y, (float*)partial, T, N, K, all, stream);
+        default: return launch_float<8>(xf, wf, bias, (float*)y, (float*)partial, T, N, K, all, stream);
     }
 }
 

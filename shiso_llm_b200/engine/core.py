@@ -152,6 +152,21 @@ def recurrence_room_bytes(plan, rows: int) -> int:
     return most
 
 
+FLOAT_PRODUCT_ROOM = 256 << 20  # csrc/gemm_simple.cu, ROOM
+
+
+def float_product_room_bytes(rows: int, longest_k: int) -> int:
+    """What a float32 product of up to ``rows`` rows and ``longest_k`` columns takes for the sums of its groups, whatever
+    its outputs' number: per 128 outputs at most 128 / tiles groups of at least 128 columns (csrc/gemm_simple.cu,
+    group_size), as long as the tiles of 64 rows are fewer than two for every one of 148 SMs (walks_all)."""
+    most = 0
+    for tiles in range(1, 128):
+        groups = min(-(-128 // tiles), longest_k // 128)
+        if groups >= 2:
+            most = max(most, 4 * groups * 128 * tiles * min(rows, 64 * (2 * 148 // tiles)))
+    return min(most, FLOAT_PRODUCT_ROOM)
+
+
 def step_buffer_bytes(plan, options: EngineOptions, dtype: torch.dtype) -> int:
     """An upper bound of what one step of ``max_num_batched_tokens`` rows allocates beside
     weights and cache: the residual stream (float32, two copies), a few activations as wide as
@@ -164,6 +179,8 @@ def step_buffer_bytes(plan, options: EngineOptions, dtype: torch.dtype) -> int:
     activations = rows * (2 * plan.hidden_size * 4 + 6 * 3 * widest * dtype.itemsize)
     logits = 2 * max(options.max_num_seqs, 1) * plan.vocab_size * 4
     workspaces = recurrence_room_bytes(plan, rows)
+    if dtype == torch.float32:
+        workspaces += float_product_room_bytes(rows, widest)
     return activations + logits + workspaces + (256 << 20)
 
 

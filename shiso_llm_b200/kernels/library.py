@@ -23,8 +23,8 @@ _SIGNATURES = {
     "shiso_gather_rows": [P, P, P, I, I, P],
     "shiso_rmsnorm": [P, P, P, P, P, I, I, I, F, P],
     "shiso_swiglu": [P, P, I, I, I, P],
-    "shiso_gemm_float_groups": [P, P, P, I, I, I],
-    "shiso_gemm_float": [P, P, P, P, P, I, I, I, P],
+    "shiso_gemm_float_groups": [P, P, P, I, I, I, I],
+    "shiso_gemm_float": [P, P, P, P, P, I, I, I, I, P],
     "shiso_gemm_simple": [P, I, P, I, P, P, I, I, I, I, P],
     "shiso_gemm_tcgen05": [P, P, P, P, I, I, I, I, I, P],
     "shiso_gemm_tcgen05_tokens64": [P, P, P, P, I, I, I, I, I, P],

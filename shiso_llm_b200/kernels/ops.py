@@ -443,10 +443,10 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype, bias: Optio
         _done(status, "linear (tcgen05)", shape=(tokens, n, k))
         return out
     if x.dtype == w.dtype == out_dtype == torch.float32:
-        groups = lib.shiso_gemm_float_groups(_ptr(x), _ptr(w), _ptr(out), tokens, n, k)
+        groups = lib.shiso_gemm_float_groups(_ptr(x), _ptr(w), _ptr(out), tokens, n, k, _sm_count())
         if groups >= 0:
             partial = torch.empty((groups, tokens, n), dtype=torch.float32, device=x.device) if groups else None
-            status = lib.shiso_gemm_float(_ptr(x), _ptr(w), _ptr(bias), _ptr(out), _ptr(partial), tokens, n, k, _stream())
+            status = lib.shiso_gemm_float(_ptr(x), _ptr(w), _ptr(bias), _ptr(out), _ptr(partial), tokens, n, k, _sm_count(), _stream())
             _done(status, "linear (float)", 2 if groups else 1, shape=(tokens, n, k))
             return out
     status = lib.shiso_gemm_simple(

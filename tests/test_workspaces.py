@@ -41,6 +41,21 @@ def test_which_steps_the_walk_takes():
     assert walk_takes(tokens=128 * 65534 + 127, seqs=1) == 1 and walk_takes(tokens=128 * 65535, seqs=1) == 0
 
 
+@pytest.mark.parametrize("sm_count", [148, 132])
+def test_float_products_stay_within_what_is_set_aside(sm_count):
+    groups_of = lambda t, n, k: library().shiso_gemm_float_groups(AT, AT, AT, t, n, k, sm_count)
+    split = 0
+    for k in (128, 256, 516, 1024, 4608, 16384):
+        for t in (1, 8, 9, 24, 100, 300, 1000, 2048, 2300, 5000, 20000):
+            room = core.float_product_room_bytes(t, k)
+            for n in (1, 100, 128, 256, 512, 900, 1024, 2048, 4608, 9216, 65536):
+                groups = groups_of(t, n, k)
+                assert groups >= 0 and 4 * groups * t * n <= room, (t, n, k, groups)
+                split += groups > 0
+    assert split > 100
+    assert groups_of(300, 1024, 1026) == -1  # rows of no multiple of four: the other kernel
+
+
 @pytest.mark.parametrize("preset", ["filulix-1b", "filulix-350m"])
 @pytest.mark.parametrize("rows", [64, 2048, 16384])
 def test_recurrences_are_set_aside_for(preset, rows):
