@@ -1,12 +1,15 @@
 // Y[T, N] = X[T, K] * W[N, K]^T (+ bias) with float accumulation on the CUDA cores.
 //
-// This is the matrix product of the true 32-bit path and the product for any
-// combination of element types the tensor-core kernels do not take (a matrix kept in
-// 32-bit beside 16-bit activations).  Every output element is accumulated by one
-// thread over k = 0 .. K-1 in ascending order with fused multiply-adds, so a row's
-// result does not depend on how many rows share the launch or where the row lies in
-// it - the property the reference calls row-exact
-// (crates/shiso-engine/src/projection.rs:972-978).  Any T, N, K >= 1.
+// gemm_float_kernel is the matrix product of the true 32-bit path where K is a multiple of four and
+// the operands lie on 16-byte boundaries.  gemm_simple_kernel is the float product otherwise, and the product
+// for any combination of element types the tensor-core kernels do not take (a matrix kept in 32-bit
+// beside 16-bit activations); T, N, K >= 1.
+//
+// Sums are fused multiply-adds over k in ascending order: gemm_simple_kernel's over k = 0 .. K-1,
+// gemm_float_kernel's within groups of K whose sums are then added up in their order.  The groups are a
+// function of N and K, so with either kernel a row's result depends neither on how many rows share the
+// launch nor on where the row lies in it - the property the reference calls row-exact
+// (crates/shiso-engine/src/projection.rs:972-978).
 #include "common.cuh"
 
 namespace {

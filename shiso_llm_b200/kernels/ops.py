@@ -405,8 +405,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: torch.dtype, bias: Optio
     """``x[T, K] @ w[N, K]^T`` with float accumulation.
 
     bfloat16 x bfloat16 runs on the tensor cores (tcgen05, accumulators in TMEM); the true
-    32-bit path and mixed types run the CUDA-core kernel, whose rows do not depend on the
-    batch."""
+    32-bit path and mixed types run the CUDA-core kernels (a float product with K in groups where the
+    operands allow 16-byte loads, else one chain a sum), whose rows do not depend on the batch."""
     _check(x, "x", None, 2)
     _check(w, "w", None, 2)
     tokens, k = x.shape
