@@ -135,6 +135,10 @@ __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
 // successor that is resident early only spins in its wait and takes registers and shared
 // memory from the CTAs that still have work to do.  The wait is a no-op for a kernel launched
 // without the attribute.  SHISO_PDL=0 turns the attribute off.
+//
+// A step's data - positions, lengths, block tables - comes from a kernel too, which loads it from the host's
+// memory and lets its successor start at once.  The step's first kernel, its embedding, is therefore launched
+// in full order (launch_in_order), and every kernel behind it may read step data ahead of its wait.
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_begin() {
@@ -148,6 +152,18 @@ SHISO_SHARED bool shiso_pdl_enabled();  // defined in elementwise.cu
 // (defined in gemm_tcgen05.cu).  The token-picking kernels hand it to the host with their
 // picks: they read it and set it back to zero.
 SHISO_SHARED int* shiso_tc_status_word();
+
+// The kernel starts when everything before it in the stream has ended and its writes can be seen.
+template <typename... KArgs, typename... Args>
+static inline void launch_in_order(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                                   Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);  // errors surface in launch_status()
+}
 
 template <typename... KArgs, typename... Args>
 static inline void launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,

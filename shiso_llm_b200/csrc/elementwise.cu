@@ -20,7 +20,8 @@ bool shiso_pdl_enabled() {
 
 // A row's token id comes from `ids`, or - where feed_index[t] >= 0 - from fed_tokens at that
 // index: the token a sampling kernel picked on the device a step earlier, which the host has
-// not seen yet.  The row is multiplied by `scale` in float (1: the row as it is).
+// not seen yet.  The row is multiplied by `scale` in float (1: the row as it is).  A step's first kernel,
+// launched in full order: common.cuh says why.
 template <typename WT>
 __global__ void embed_kernel(const int* __restrict__ ids, const int* __restrict__ feed_index,
                              const int* fed_tokens, const WT* __restrict__ table,
@@ -44,9 +45,9 @@ SHISO_API int shiso_embed_scaled(const int* ids, const int* feed_index, const in
     if ((feed_index == nullptr) != (fed_tokens == nullptr)) return SHISO_ERR_SHAPE;
     const int threads = hidden >= 1024 ? 256 : 128;
     if (table_dtype == SHISO_F32)
-        launch_kernel(embed_kernel<float>, tokens, threads, 0, stream, ids, feed_index, fed_tokens, (const float*)table, out, hidden, vocab, scale);
+        launch_in_order(embed_kernel<float>, tokens, threads, 0, stream, ids, feed_index, fed_tokens, (const float*)table, out, hidden, vocab, scale);
     else if (table_dtype == SHISO_BF16)
-        launch_kernel(embed_kernel<__nv_bfloat16>, tokens, threads, 0, stream, ids, feed_index, fed_tokens, (const __nv_bfloat16*)table, out, hidden, vocab, scale);
+        launch_in_order(embed_kernel<__nv_bfloat16>, tokens, threads, 0, stream, ids, feed_index, fed_tokens, (const __nv_bfloat16*)table, out, hidden, vocab, scale);
     else
         return SHISO_ERR_DTYPE;
     return launch_status();

@@ -21,7 +21,8 @@ __device__ __forceinline__ int step_token(const int* ids, const int* feed_index,
 
 // x_t = scale * E[id_t] + B[(id_{t-1} * mul_prev + id_t * mul_cur) mod buckets]; B[buckets] for a
 // sequence's first token.  The previous token of a portion's first row is what the request's
-// slot holds (token + 1).  The slots are written by the kernel below, after this one.
+// slot holds (token + 1).  The slots are written by the kernel below, after this one.  A step's first
+// kernel, launched in full order: common.cuh says why.
 template <typename WT>
 __global__ void embed_hashed_pair_kernel(const int* __restrict__ ids, const int* __restrict__ feed_index, const int* fed_tokens,
                                          const WT* __restrict__ table, const WT* __restrict__ pair_table,
@@ -64,11 +65,11 @@ SHISO_API int shiso_embed_hashed_pair(const int* ids, const int* feed_index, con
     if ((feed_index == nullptr) != (fed_tokens == nullptr) || buckets <= 0) return SHISO_ERR_SHAPE;
     const int threads = hidden >= 1024 ? 256 : 128;
     if (table_dtype == SHISO_F32)
-        launch_kernel(embed_hashed_pair_kernel<float>, tokens, threads, 0, stream, ids, feed_index, fed_tokens, (const float*)table,
+        launch_in_order(embed_hashed_pair_kernel<float>, tokens, threads, 0, stream, ids, feed_index, fed_tokens, (const float*)table,
                       (const float*)pair_table, seq_of_token, q_start, start_pos, slots, (const int*)state, state_stride, out,
                       hidden, vocab, scale, buckets, mul_prev, mul_cur);
     else if (table_dtype == SHISO_BF16)
-        launch_kernel(embed_hashed_pair_kernel<__nv_bfloat16>, tokens, threads, 0, stream, ids, feed_index, fed_tokens,
+        launch_in_order(embed_hashed_pair_kernel<__nv_bfloat16>, tokens, threads, 0, stream, ids, feed_index, fed_tokens,
                       (const __nv_bfloat16*)table, (const __nv_bfloat16*)pair_table, seq_of_token, q_start, start_pos, slots,
                       (const int*)state, state_stride, out, hidden, vocab, scale, buckets, mul_prev, mul_cur);
     else
