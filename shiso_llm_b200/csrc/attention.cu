@@ -40,9 +40,9 @@ struct UnitRegs {
 
 template <typename AT, int HD_MAX>
 __global__ void __launch_bounds__(WARPS * 32)
-qk_norm_rope_store_kernel(const AT* __restrict__ qkv, const float* __restrict__ q_w, const float* __restrict__ k_w,
-                          const float* __restrict__ inv_freq, const int* __restrict__ positions,
-                          const int* __restrict__ seq_of_token, const int* __restrict__ block_table,
+qk_norm_rope_store_kernel(const AT* qkv, const float* __restrict__ q_w, const float* __restrict__ k_w,
+                          const float* __restrict__ inv_freq, const int* positions,
+                          const int* seq_of_token, const int* block_table,
                           int table_width, AT* __restrict__ k_cache, AT* __restrict__ v_cache,
                           AT* __restrict__ q_out, int tokens, int heads, int kv_heads, int head_dim,
                           int rotary_dim, int page_size, float eps, int store, int per_warp, int interleaved) {
@@ -155,10 +155,10 @@ qk_norm_rope_store_kernel(const AT* __restrict__ qkv, const float* __restrict__ 
 // and the angle's sine and cosine serve all of them.  At 2,048 rows the kernel above moved its
 // 25 MB at 1.1 TB/s, most of its time being instructions per byte.
 __global__ void __launch_bounds__(WARPS * 32)
-qk_norm_rope_store64_kernel(const __nv_bfloat16* __restrict__ qkv, const float* __restrict__ q_w,
+qk_norm_rope_store64_kernel(const __nv_bfloat16* qkv, const float* __restrict__ q_w,
                             const float* __restrict__ k_w, const float* __restrict__ inv_freq,
-                            const int* __restrict__ positions, const int* __restrict__ seq_of_token,
-                            const int* __restrict__ block_table, int table_width, __nv_bfloat16* __restrict__ k_cache,
+                            const int* positions, const int* seq_of_token,
+                            const int* block_table, int table_width, __nv_bfloat16* __restrict__ k_cache,
                             __nv_bfloat16* __restrict__ v_cache, __nv_bfloat16* __restrict__ q_out, int tokens, int heads,
                             int kv_heads, int page_size, float eps, int store, int groups_per_warp) {
     pdl_begin();
@@ -266,9 +266,9 @@ qk_norm_rope_store64_kernel(const __nv_bfloat16* __restrict__ qkv, const float* 
 
 template <typename AT>
 __global__ void __launch_bounds__(WARPS * 32)
-paged_attention_kernel(const AT* __restrict__ q, const AT* __restrict__ k_cache, const AT* __restrict__ v_cache,
-                       const int* __restrict__ block_table, int table_width, const int* __restrict__ positions,
-                       const int* __restrict__ seq_of_token, AT* __restrict__ out, int tokens, int heads,
+paged_attention_kernel(const AT* q, const AT* k_cache, const AT* v_cache,
+                       const int* block_table, int table_width, const int* positions,
+                       const int* seq_of_token, AT* __restrict__ out, int tokens, int heads,
                        int kv_heads, int head_dim, int page_size, float scale, int window) {
     pdl_wait();
     __shared__ float q_s[WARPS][MAX_HEAD_DIM];

@@ -263,7 +263,7 @@ decode_split_kernel(DecodeArgs a) {
     }
 }
 
-__global__ void decode_merge_kernel(const float* __restrict__ partial, __nv_bfloat16* __restrict__ out, int heads,
+__global__ void decode_merge_kernel(const float* partial, __nv_bfloat16* __restrict__ out, int heads,
                                     int head_dim, int splits) {
     pdl_begin();
     const int h = blockIdx.x, t = blockIdx.y;

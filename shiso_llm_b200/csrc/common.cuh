@@ -136,6 +136,11 @@ __device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b) {
 // memory from the CTAs that still have work to do.  The wait is a no-op for a kernel launched
 // without the attribute.  SHISO_PDL=0 turns the attribute off.
 //
+// What a kernel before may have written is read through pointers without __restrict__ const: such loads
+// count as unchanging for the whole kernel and may be moved ahead of the wait (an index read that
+// way reached past its array).  For the same reason no pointer that is read and written has __restrict__.  Weights
+// are no kernel's output, and what a kernel only writes cannot be read early: these may have it.
+//
 // A step's data - positions, lengths, block tables - comes from a kernel too, which loads it from the host's
 // memory and lets its successor start at once.  The step's first kernel, its embedding, is therefore launched
 // in full order (launch_in_order), and every kernel behind it may read step data ahead of its wait.

@@ -656,7 +656,7 @@ int launch_delta_step(const StepArgs& a, int num_seqs, cudaStream_t stream) {
 // power of two) a (row, head), each with four neighbouring columns at a time (N = 4) or one.
 template <typename AT, int N>
 __global__ void __launch_bounds__(256)
-delta_output_kernel(const float* __restrict__ x, const AT* __restrict__ gate, long long gate_ld, const float* __restrict__ w,
+delta_output_kernel(const float* x, const AT* gate, long long gate_ld, const float* __restrict__ w,
                     AT* __restrict__ out, long long out_ld, int tokens, int heads, int vdim, int group, float eps) {
     pdl_begin();
     const long long item = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / group;

@@ -25,7 +25,7 @@ template <int N> __device__ __forceinline__ void load_cols(const float* p, float
 }
 
 template <typename AT, int N>
-__global__ void __launch_bounds__(256) map_difference_kernel(const DifferenceArgs a, const AT* __restrict__ gate, AT* __restrict__ out) {
+__global__ void __launch_bounds__(256) map_difference_kernel(const DifferenceArgs a, const AT* gate, AT* __restrict__ out) {
     pdl_begin();
     const long long item = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / a.group;
     const int sub = threadIdx.x % a.group;

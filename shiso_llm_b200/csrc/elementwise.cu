@@ -23,7 +23,7 @@ bool shiso_pdl_enabled() {
 // not seen yet.  The row is multiplied by `scale` in float (1: the row as it is).  A step's first kernel,
 // launched in full order: common.cuh says why.
 template <typename WT>
-__global__ void embed_kernel(const int* __restrict__ ids, const int* __restrict__ feed_index,
+__global__ void embed_kernel(const int* ids, const int* feed_index,
                              const int* fed_tokens, const WT* __restrict__ table,
                              float* __restrict__ out, int hidden, int vocab, float scale) {
     pdl_begin();
@@ -58,7 +58,7 @@ SHISO_API int shiso_embed(const int* ids, const int* feed_index, const int* fed_
     return shiso_embed_scaled(ids, feed_index, fed_tokens, table, table_dtype, out, tokens, hidden, vocab, 1.0f, stream);
 }
 
-__global__ void gather_rows_kernel(const float* __restrict__ src, const int* __restrict__ rows,
+__global__ void gather_rows_kernel(const float* src, const int* rows,
                                    float* __restrict__ out, int hidden) {
     pdl_begin();
     const float* s = src + (size_t)rows[blockIdx.x] * hidden;
@@ -80,8 +80,8 @@ SHISO_API int shiso_gather_rows(const float* src, const int* rows, float* out, i
 // row blockIdx.x of the output is the norm of source row rows[blockIdx.x] and the
 // residual is left alone (used for the final norm of the wanted rows only).
 template <typename AT>
-__global__ void rmsnorm_kernel(float* __restrict__ residual, const AT* __restrict__ delta,
-                               const int* __restrict__ rows, const float* __restrict__ w,
+__global__ void rmsnorm_kernel(float* residual, const AT* delta,
+                               const int* rows, const float* __restrict__ w,
                                AT* __restrict__ out, int hidden, float eps) {
     pdl_begin();
     __shared__ float scratch[33];
@@ -297,7 +297,7 @@ SHISO_API int shiso_rmsnorm(float* residual, const void* delta, const int* rows,
 // --------------------------------------------------------------------------- SwiGLU
 
 template <typename AT>
-__global__ void swiglu_kernel(const AT* __restrict__ gate_up, AT* __restrict__ out, int inter, long long total) {
+__global__ void swiglu_kernel(const AT* gate_up, AT* __restrict__ out, int inter, long long total) {
     pdl_begin();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;

@@ -379,7 +379,7 @@ enum { ROUTE_SOFTMAX = 0, ROUTE_SIGMOID = 1, ROUTE_CHOSEN_SOFTMAX = 2 };
 // their experts the `top` largest choice scores win (the lower index on a tie); weight = score
 // (/ (the chosen scores' sum + renorm_eps)) * scale.  ROUTE_CHOSEN_SOFTMAX: the scores are the logits
 // themselves, and the weights the softmax over the chosen ones, times scale.  Rows of logits are `ld` apart.
-__global__ void moe_route_kernel(const float* __restrict__ logits, long long ld, const float* __restrict__ correction,
+__global__ void moe_route_kernel(const float* logits, long long ld, const float* __restrict__ correction,
                                  int* __restrict__ ids, float* __restrict__ weights, int tokens, int experts, int top,
                                  int group_count, int group_keep, float scale, int scoring, int renormalize, float renorm_eps) {
     pdl_begin();
@@ -489,14 +489,14 @@ __global__ void moe_zero_kernel(int* __restrict__ counts, int experts) {
     for (int e = threadIdx.x; e < experts; e += blockDim.x) counts[e] = 0;
 }
 
-__global__ void moe_count_kernel(const int* __restrict__ ids, int* __restrict__ counts, int* __restrict__ rank, int total) {
+__global__ void moe_count_kernel(const int* ids, int* counts, int* __restrict__ rank, int total, int experts) {
     pdl_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < total) rank[i] = atomicAdd(&counts[ids[i]], 1);
+    if (i < total) rank[i] = atomicAdd(&counts[min(max(ids[i], 0), experts - 1)], 1);  // (never past the counts, whatever the ids)
 }
 
 // place[i] = first row of the choice's expert + its rank there; source[place] = i
-__global__ void moe_place_kernel(const int* __restrict__ ids, const int* __restrict__ counts, const int* __restrict__ rank,
+__global__ void moe_place_kernel(const int* ids, const int* counts, const int* rank,
                                  int* __restrict__ place, int* __restrict__ source, int total, int experts) {
     pdl_begin();
     __shared__ int first[MOE_MAX_EXPERTS];
@@ -510,7 +510,7 @@ __global__ void moe_place_kernel(const int* __restrict__ ids, const int* __restr
     __syncthreads();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
-    const int p = first[ids[i]] + rank[i];
+    const int p = first[min(max(ids[i], 0), experts - 1)] + rank[i];
     place[i] = p;
     source[p] = i;
 }
@@ -518,9 +518,9 @@ __global__ void moe_place_kernel(const int* __restrict__ ids, const int* __restr
 // out[t] = extra[t] (* sigmoid(extra_gate[t])) + sum_j weights[t, j] * y[place[t * top + j]], the choices in
 // their order (with weigh_input the weight has gone into the expert's input and counts no more here); a choice whose id is `experts` or more is an identity expert: it adds weights[t, j] * x[t].
 template <typename AT>
-__global__ void moe_combine_kernel(const float* __restrict__ y, const int* __restrict__ place, const float* __restrict__ weights,
-                                   const int* __restrict__ ids, const AT* __restrict__ x, const AT* __restrict__ extra,
-                                   const float* __restrict__ extra_gate, long long extra_gate_ld, AT* __restrict__ out, int tokens,
+__global__ void moe_combine_kernel(const float* y, const int* place, const float* weights,
+                                   const int* ids, const AT* x, const AT* extra,
+                                   const float* extra_gate, long long extra_gate_ld, AT* __restrict__ out, int tokens,
                                    int hidden, int top, int experts, int weigh_input) {
     pdl_begin();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -563,7 +563,7 @@ SHISO_API int shiso_routed_experts(const void* x, int act_dtype, const int* ids,
     int* place = rank + total;
     int* source = place + total;
     launch_kernel(moe_zero_kernel, 1, 256, 0, stream, counts, outputs);
-    launch_kernel(moe_count_kernel, ceil_div_u(total, 256), 256, 0, stream, ids, counts, rank, total);
+    launch_kernel(moe_count_kernel, ceil_div_u(total, 256), 256, 0, stream, ids, counts, rank, total, outputs);
     launch_kernel(moe_place_kernel, ceil_div_u(total, 256), 256, 0, stream, ids, (const int*)counts, (const int*)rank, place, source,
                   total, outputs);
     int status = launch_status();

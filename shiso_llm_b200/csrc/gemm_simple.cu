@@ -18,7 +18,7 @@ constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
 
 template <typename WT, typename XT, typename OT>
 __global__ void __launch_bounds__(256)
-gemm_simple_kernel(const XT* __restrict__ x, const WT* __restrict__ w, const float* __restrict__ bias,
+gemm_simple_kernel(const XT* x, const WT* __restrict__ w, const float* __restrict__ bias,
                    OT* __restrict__ y, int T, int N, int K) {
     pdl_wait();
     __shared__ float xs[BK][BM + 4];
@@ -101,7 +101,7 @@ constexpr int PN = 128, PK = 16, P_THREADS = 128;
 // group blockIdx.z, whose sums go to partial[blockIdx.z][T][N].
 template <int TM, bool ALL>
 __global__ void __launch_bounds__(P_THREADS, TM == 8 ? 2 : 4)
-gemm_float_kernel(const float* __restrict__ x, const float* __restrict__ w, const float* __restrict__ bias, float* __restrict__ y,
+gemm_float_kernel(const float* x, const float* __restrict__ w, const float* __restrict__ bias, float* __restrict__ y,
                   float* __restrict__ partial, int T, int N, int K, int group) {
     constexpr int PM = 8 * TM, XROW = PM + 4, WROW = PN + 4;
     __shared__ __align__(16) float xs[2][PK][XROW], ws[2][PK][WROW];
@@ -233,7 +233,7 @@ gemm_float_kernel(const float* __restrict__ x, const float* __restrict__ w, cons
 }
 
 // y = the groups' sums in their order (+ bias).
-__global__ void __launch_bounds__(256) gemm_float_join_kernel(const float* __restrict__ partial, const float* __restrict__ bias,
+__global__ void __launch_bounds__(256) gemm_float_join_kernel(const float* partial, const float* __restrict__ bias,
                                                               float* __restrict__ y, long long count, int N, int groups) {
     pdl_begin();
     const long long at = ((long long)blockIdx.x * 256 + threadIdx.x) * 4;

@@ -53,8 +53,8 @@ template <typename AT, int E> __device__ __forceinline__ void la_load(const AT* 
 // RV: latent entries a lane sums (rank <= 32 RV).  VEC: the cached rows are read 16 bytes at a time.
 template <typename AT, int RV, bool VEC>
 __global__ void __launch_bounds__(LA_WARPS * 32) latent_attention_kernel(
-    const AT* __restrict__ q, const AT* __restrict__ cache, const int* __restrict__ block_table, int table_width,
-    const int* __restrict__ positions, const int* __restrict__ seq_of_token, AT* __restrict__ out, float* __restrict__ scratch,
+    const AT* q, const AT* cache, const int* block_table, int table_width,
+    const int* positions, const int* seq_of_token, AT* __restrict__ out, float* __restrict__ scratch,
     int heads, int rank, int width, int page_size, float scale, int shares) {
     extern __shared__ float sm[];
     float* sq = sm;                                  // [LA_HEADS][width], times scale
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(LA_WARPS * 32) latent_attention_kernel(
 
 // The shares of a (row, head) in share order: [maximum, sum, rank sums] each.
 template <typename AT>
-__global__ void latent_attention_merge_kernel(const float* __restrict__ scratch, AT* __restrict__ out, int rank, int shares) {
+__global__ void latent_attention_merge_kernel(const float* scratch, AT* __restrict__ out, int rank, int shares) {
     pdl_begin();
     const float* parts = scratch + (size_t)blockIdx.x * shares * (rank + 2);
     float top = -INFINITY;

@@ -44,9 +44,9 @@ enum { MA_MASK_WINDOW = 0, MA_MASK_CHUNK = 1 };
 
 template <typename AT>
 __global__ void __launch_bounds__(MA_WARPS * 32)
-head_prepare_store_kernel(AT* __restrict__ proj, long long ld, int q_col, int k_col, int v_col, const float* __restrict__ q_w,
-                          const float* __restrict__ k_w, const float* __restrict__ inv_freq, const int* __restrict__ positions,
-                          const int* __restrict__ seq_of_token, const int* __restrict__ table, int table_width,
+head_prepare_store_kernel(AT* proj, long long ld, int q_col, int k_col, int v_col, const float* __restrict__ q_w,
+                          const float* __restrict__ k_w, const float* __restrict__ inv_freq, const int* positions,
+                          const int* seq_of_token, const int* table, int table_width,
                           AT* __restrict__ k_cache, AT* __restrict__ v_cache, int heads, int kv_heads, int v_heads, int dim, int vdim,
                           int rotary_dim, int page_size, float eps, float magnitude, int norm_mode, int store) {
     __shared__ float buf[MA_WARPS][MA_MAX_DIM];
@@ -140,9 +140,9 @@ head_prepare_store_kernel(AT* __restrict__ proj, long long ld, int q_col, int k_
 constexpr int MA_VEC_THREADS = 256;
 
 __global__ void __launch_bounds__(MA_VEC_THREADS)
-head_prepare_store_vec_kernel(__nv_bfloat16* __restrict__ proj, long long ld, int q_col, int k_col, int v_col,
+head_prepare_store_vec_kernel(__nv_bfloat16* proj, long long ld, int q_col, int k_col, int v_col,
                               const float* __restrict__ q_w, const float* __restrict__ k_w, const float* __restrict__ inv_freq,
-                              const int* __restrict__ positions, const int* __restrict__ seq_of_token, const int* __restrict__ table,
+                              const int* positions, const int* seq_of_token, const int* table,
                               int table_width, __nv_bfloat16* __restrict__ k_cache, __nv_bfloat16* __restrict__ v_cache, int heads,
                               int kv_heads, int v_heads, int dim, int vdim, int rotary_dim, int page_size, float eps, float magnitude,
                               int norm_mode, int store, int group) {
@@ -239,7 +239,7 @@ __device__ __forceinline__ float2 ma_load_pair(const __nv_bfloat16* p) {
 }
 
 // q . key over `dim` channels; 16-byte loads of the key where its rows allow them.
-__device__ __forceinline__ float ma_dot(const float* __restrict__ q, const float* __restrict__ key, int dim, bool wide) {
+__device__ __forceinline__ float ma_dot(const float* q, const float* key, int dim, bool wide) {
     float dot = 0.0f;
     if (wide) {
 #pragma unroll 4
@@ -252,7 +252,7 @@ __device__ __forceinline__ float ma_dot(const float* __restrict__ q, const float
     }
     return dot;
 }
-__device__ __forceinline__ float ma_dot(const float* __restrict__ q, const __nv_bfloat16* __restrict__ key, int dim, bool wide) {
+__device__ __forceinline__ float ma_dot(const float* q, const __nv_bfloat16* key, int dim, bool wide) {
     float dot = 0.0f;
     if (wide) {
 #pragma unroll 8
@@ -300,7 +300,7 @@ __device__ __forceinline__ void ma_lists(const MaskedArgs& a, int pos, int& kept
 // A warp folds 32 keys (positions first + base ..) into its running result: a lane takes a key and
 // forms the whole dot product; the lanes then share the value channels.
 template <typename AT, bool SIGMOID>
-__device__ __forceinline__ void ma_fold(const MaskedArgs& a, const AT* __restrict__ k_cache, const AT* __restrict__ v_cache,
+__device__ __forceinline__ void ma_fold(const MaskedArgs& a, const AT* k_cache, const AT* v_cache,
                                         const int* pages, int first, int count, int base, int kv_head, const float* q, float bias,
                                         float& running_max, float& running_sum, float (&acc)[MA_PAIRS][2], int lane,
                                         float* run_weight, long long* run_row) {
@@ -379,8 +379,8 @@ template <typename AT> struct MaskedOut {
 
 template <typename AT, bool SIGMOID>
 __global__ void __launch_bounds__(MA_WARPS * 32)
-masked_attention_kernel(const AT* __restrict__ q, const AT* __restrict__ k_cache, const AT* __restrict__ v_cache, void* out,
-                        const AT* __restrict__ gate, MaskedArgs a) {
+masked_attention_kernel(const AT* q, const AT* k_cache, const AT* v_cache, void* out,
+                        const AT* gate, MaskedArgs a) {
     __shared__ float sq[MA_MAX_DIM];
     __shared__ float run_weight[MA_WARPS][32];
     __shared__ long long run_row[MA_WARPS][32];
@@ -486,7 +486,7 @@ masked_attention_kernel(const AT* __restrict__ q, const AT* __restrict__ k_cache
 // Adds up the shares of a (row, head) in split order; softmax shares are brought to one maximum first.
 template <typename AT, bool SIGMOID>
 __global__ void __launch_bounds__(128)
-masked_attention_merge_kernel(void* out, const AT* __restrict__ gate, MaskedArgs a) {
+masked_attention_merge_kernel(void* out, const AT* gate, MaskedArgs a) {
     pdl_begin();
     const int t = blockIdx.x / a.heads, head = blockIdx.x % a.heads;
     const float* parts = a.scratch + (size_t)blockIdx.x * a.splits * (a.vdim + 2);

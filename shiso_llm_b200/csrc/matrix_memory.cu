@@ -113,7 +113,7 @@ struct OutputArgs {
 
 // `group` lanes (a power of two) a (row, head), each with N neighbouring columns at a time.
 template <typename AT, int N>
-__global__ void __launch_bounds__(256) memory_output_kernel(const OutputArgs a, const AT* __restrict__ gate, AT* __restrict__ out) {
+__global__ void __launch_bounds__(256) memory_output_kernel(const OutputArgs a, const AT* gate, AT* __restrict__ out) {
     pdl_begin();
     const long long item = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / a.group;
     const int sub = threadIdx.x % a.group;

@@ -15,7 +15,7 @@
 namespace {
 
 template <typename AT>
-__global__ void norm_into_kernel(float* __restrict__ residual, const AT* __restrict__ y, const float* __restrict__ w, AT* __restrict__ out,
+__global__ void norm_into_kernel(float* residual, const AT* y, const float* __restrict__ w, AT* __restrict__ out,
                                  int hidden, float eps) {
     __shared__ float scratch[33];
     pdl_begin();
@@ -35,7 +35,7 @@ __global__ void norm_into_kernel(float* __restrict__ residual, const AT* __restr
 }
 
 template <typename AT>
-__global__ void polynorm_kernel(const AT* __restrict__ z, long long z_ld, const float* __restrict__ coefficients, AT* __restrict__ out,
+__global__ void polynorm_kernel(const AT* z, long long z_ld, const float* __restrict__ coefficients, AT* __restrict__ out,
                                 int width, float eps) {
     __shared__ float scratch[33];
     pdl_begin();
@@ -81,7 +81,7 @@ __device__ __forceinline__ uint4 pack8(const float (&v)[8]) {
     return *reinterpret_cast<uint4*>(h);
 }
 
-__global__ void norm_into_vec_kernel(float* __restrict__ residual, const __nv_bfloat16* __restrict__ y, const float* __restrict__ w,
+__global__ void norm_into_vec_kernel(float* residual, const __nv_bfloat16* y, const float* __restrict__ w,
                                      __nv_bfloat16* __restrict__ out, int hidden, float eps) {
     __shared__ float scratch[33];
     pdl_begin();
@@ -216,7 +216,7 @@ template <int N> __device__ __forceinline__ void pair_store(__nv_bfloat16* p, co
 
 // PAIR false: there is no second branch (right, wb unused).
 template <typename AT, int N, bool PAIR>
-__global__ void normed_pair_kernel(const NormedPairArgs a, const AT* __restrict__ left, const AT* __restrict__ right, AT* __restrict__ out) {
+__global__ void normed_pair_kernel(const NormedPairArgs a, const AT* left, const AT* right, AT* __restrict__ out) {
     __shared__ float scratch[33];
     extern __shared__ __align__(16) float row_cache[];
     pdl_begin();

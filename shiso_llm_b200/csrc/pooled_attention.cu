@@ -19,9 +19,9 @@
 #include "common.cuh"
 
 template <typename AT>
-__global__ void store_kv_kernel(const AT* __restrict__ k, long long k_ld, const AT* __restrict__ v, long long v_ld,
-                                const int* __restrict__ positions, const int* __restrict__ seq_of_token,
-                                const int* __restrict__ table, int table_width, AT* __restrict__ k_cache, AT* __restrict__ v_cache,
+__global__ void store_kv_kernel(const AT* k, long long k_ld, const AT* v, long long v_ld,
+                                const int* positions, const int* seq_of_token,
+                                const int* table, int table_width, AT* __restrict__ k_cache, AT* __restrict__ v_cache,
                                 int kv_heads, int dim, int vdim, int page_size) {
     pdl_begin();
     const int t = blockIdx.x;
@@ -125,7 +125,7 @@ __device__ __forceinline__ float2 load_pair(const __nv_bfloat16* p) {
 }
 
 // q . key over `dim` channels; 16-byte loads of the key where its rows allow them.
-__device__ __forceinline__ float dot_key(const float* __restrict__ q, const float* __restrict__ key, int dim, bool wide) {
+__device__ __forceinline__ float dot_key(const float* q, const float* key, int dim, bool wide) {
     float dot = 0.0f;
     if (wide) {
 #pragma unroll 4
@@ -138,7 +138,7 @@ __device__ __forceinline__ float dot_key(const float* __restrict__ q, const floa
     }
     return dot;
 }
-__device__ __forceinline__ float dot_key(const float* __restrict__ q, const __nv_bfloat16* __restrict__ key, int dim, bool wide) {
+__device__ __forceinline__ float dot_key(const float* q, const __nv_bfloat16* key, int dim, bool wide) {
     float dot = 0.0f;
     if (wide) {
 #pragma unroll 4
@@ -161,7 +161,7 @@ __device__ __forceinline__ float dot_key(const float* __restrict__ q, const __nv
 // its running softmax: a lane takes a key and forms the whole dot product; the lanes then share
 // the value channels.
 template <typename CT>
-__device__ __forceinline__ void fold_chunk(const CT* __restrict__ k_cache, const CT* __restrict__ v_cache, const int* pages,
+__device__ __forceinline__ void fold_chunk(const CT* k_cache, const CT* v_cache, const int* pages,
                                            int first, int count, int base, int page_size, int kv_heads, int kv_head, int dim,
                                            int vdim, const float* q, float scale, float& running_max, float& running_sum,
                                            float (&acc)[PWA_PAIRS][2], int lane, float* run_weight, long long* run_row) {
@@ -225,10 +225,10 @@ __device__ __forceinline__ void fold_chunk(const CT* __restrict__ k_cache, const
 // position only.
 template <typename AT>
 __global__ void __launch_bounds__(PWA_WARPS * 32)
-pooled_window_attention_kernel(const AT* __restrict__ q, long long q_ld, const AT* __restrict__ k_cache,
-                               const AT* __restrict__ v_cache, const int* __restrict__ table, const float* __restrict__ pooled_k,
-                               const float* __restrict__ pooled_v, const int* __restrict__ pooled_table, int table_width,
-                               const int* __restrict__ positions, const int* __restrict__ seq_of_token, AT* out,
+pooled_window_attention_kernel(const AT* q, long long q_ld, const AT* k_cache,
+                               const AT* v_cache, const int* table, const float* pooled_k,
+                               const float* pooled_v, const int* pooled_table, int table_width,
+                               const int* positions, const int* seq_of_token, AT* out,
                                long long out_ld, int heads, int kv_heads, int dim, int vdim,
                                int page_size, float scale, int window, int pool, float out_scale) {
     __shared__ float sq[PWA_MAX_DIM];
@@ -303,10 +303,10 @@ pooled_window_attention_kernel(const AT* __restrict__ q, long long q_ld, const A
 // blocks (its position / pool at most), so a warp takes a (row, head) by itself, eight to a CTA.
 template <typename AT>
 __global__ void __launch_bounds__(PWA_WARPS * 32)
-pooled_blocks_merge_kernel(const AT* __restrict__ q, long long q_ld, const float* __restrict__ pooled_k,
-                           const float* __restrict__ pooled_v, const int* __restrict__ pooled_table, int table_width,
-                           const int* __restrict__ positions, const int* __restrict__ seq_of_token, AT* out, long long out_ld,
-                           const float* __restrict__ seen, int tokens, int heads, int kv_heads, int dim, int vdim, int page_size,
+pooled_blocks_merge_kernel(const AT* q, long long q_ld, const float* pooled_k,
+                           const float* pooled_v, const int* pooled_table, int table_width,
+                           const int* positions, const int* seq_of_token, AT* out, long long out_ld,
+                           const float* seen, int tokens, int heads, int kv_heads, int dim, int vdim, int page_size,
                            float scale, int window, int pool, float out_scale) {
     __shared__ float sq[PWA_WARPS][PWA_MAX_DIM];
     __shared__ float run_weight[PWA_WARPS][32];

@@ -39,8 +39,8 @@ __device__ __forceinline__ float turned(float x, float other, float cs, float sn
 // Unit RMS over a head's value channels, times weight, silu(gate) and a constant: what follows the
 // recurrence when its outputs were left unnormalised.  A warp per (row, head).
 template <typename AT>
-__global__ void unit_rms_gate_kernel(const float* __restrict__ raw, const AT* __restrict__ gate, long long gate_ld,
-                                     const float* __restrict__ out_weight, AT* __restrict__ out, long long out_ld, int tokens,
+__global__ void unit_rms_gate_kernel(const float* raw, const AT* gate, long long gate_ld,
+                                     const float* out_weight, AT* __restrict__ out, long long out_ld, int tokens,
                                      int heads, int vdim, float eps, float out_scale) {
     pdl_begin();
     const int lane = threadIdx.x & 31;
@@ -83,8 +83,8 @@ __device__ __forceinline__ void store_two(__nv_bfloat16* p, float x, float y) {
 // The same bits with two channels of every 32 a lane, 16 lanes to a row of a head: lane l adds the squares up
 // for the lanes 2 l and 2 l + 1 of the kernel above.
 template <typename AT, int VDIM>
-__global__ void unit_rms_gate_pairs_kernel(const float* __restrict__ raw, const AT* __restrict__ gate, long long gate_ld,
-                                           const float* __restrict__ out_weight, AT* __restrict__ out, long long out_ld, int tokens,
+__global__ void unit_rms_gate_pairs_kernel(const float* raw, const AT* gate, long long gate_ld,
+                                           const float* out_weight, AT* __restrict__ out, long long out_ld, int tokens,
                                            int heads, float eps, float out_scale) {
     pdl_begin();
     constexpr int PAIRS = VDIM / 32;

@@ -14,8 +14,8 @@
 // (x - mean) / sqrt(mean((x - mean)^2) + eps) * w.  One block per output row; the row is kept
 // in shared memory so that the variance is taken from the deviations themselves.
 template <typename AT>
-__global__ void add_layernorm_kernel(float* __restrict__ residual, const AT* __restrict__ d1, const AT* __restrict__ d2,
-                                     const int* __restrict__ rows, const float* __restrict__ w, AT* __restrict__ out,
+__global__ void add_layernorm_kernel(float* residual, const AT* d1, const AT* d2,
+                                     const int* rows, const float* __restrict__ w, AT* __restrict__ out,
                                      int hidden, float eps) {
     pdl_begin();
     __shared__ float scratch[33];
@@ -77,7 +77,7 @@ enum { SHISO_GATE_NONE = 0, SHISO_GATE_SILU_BEFORE = 1, SHISO_GATE_SIGMOID_AFTER
 // One block per (row, group): the group's columns times silu(gate) (mode 1), divided by their
 // root mean square, times w, times sigmoid(gate) (mode 2).
 template <typename XT, typename AT>
-__global__ void group_rmsnorm_kernel(const XT* __restrict__ x, long long x_ld, const AT* __restrict__ gate, long long gate_ld,
+__global__ void group_rmsnorm_kernel(const XT* x, long long x_ld, const AT* gate, long long gate_ld,
                                      const float* __restrict__ w, AT* __restrict__ out, int width, int groups, int mode, float eps) {
     pdl_begin();
     __shared__ float scratch[33];
@@ -146,10 +146,10 @@ SHISO_API int shiso_group_rmsnorm(const void* x, int x_dtype, long long x_ld, co
 // constant); a run that crosses into another sequence takes its rows one by one.  The slot is
 // read here and written by the kernel below.
 template <typename AT>
-__global__ void causal_conv_kernel(const AT* __restrict__ x, long long x_ld, const float* __restrict__ taps,
-                                   const float* __restrict__ bias, const float* __restrict__ state, long long slot_stride,
-                                   const int* __restrict__ seq_of_token, const int* __restrict__ q_start,
-                                   const int* __restrict__ state_slots, AT* __restrict__ y, int tokens, int channels, int n_taps,
+__global__ void causal_conv_kernel(const AT* x, long long x_ld, const float* __restrict__ taps,
+                                   const float* __restrict__ bias, const float* state, long long slot_stride,
+                                   const int* seq_of_token, const int* q_start,
+                                   const int* state_slots, AT* __restrict__ y, int tokens, int channels, int n_taps,
                                    int silu) {
     pdl_begin();
     constexpr int M = SHISO_CONV_MAX_TAPS;
@@ -213,9 +213,9 @@ __global__ void causal_conv_kernel(const AT* __restrict__ x, long long x_ld, con
 // is rounded to 2^-9).
 template <int TAPS>
 __global__ void __launch_bounds__(128)
-causal_conv_vec_kernel(const __nv_bfloat16* __restrict__ x, long long x_ld, const float* __restrict__ taps, const float* __restrict__ bias,
-                       const float* __restrict__ state, long long slot_stride, const int* __restrict__ seq_of_token,
-                       const int* __restrict__ q_start, const int* __restrict__ state_slots, __nv_bfloat16* __restrict__ y, int tokens,
+causal_conv_vec_kernel(const __nv_bfloat16* x, long long x_ld, const float* __restrict__ taps, const float* __restrict__ bias,
+                       const float* state, long long slot_stride, const int* seq_of_token,
+                       const int* q_start, const int* state_slots, __nv_bfloat16* __restrict__ y, int tokens,
                        int channels, int silu, int run_rows) {
     pdl_begin();
     const int groups = channels >> 3;
@@ -293,8 +293,8 @@ causal_conv_vec_kernel(const __nv_bfloat16* __restrict__ x, long long x_ld, cons
 // slot held where the portion is shorter).  A thread per (sequence, channel) walks the L-1 rows
 // in an order that never reads a value it has overwritten.
 template <typename AT>
-__global__ void causal_conv_state_kernel(const AT* __restrict__ x, long long x_ld, float* __restrict__ state, long long slot_stride,
-                                         const int* __restrict__ q_start, const int* __restrict__ state_slots, int num_seqs,
+__global__ void causal_conv_state_kernel(const AT* x, long long x_ld, float* state, long long slot_stride,
+                                         const int* q_start, const int* state_slots, int num_seqs,
                                          int channels, int n_taps) {
     pdl_wait();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -353,8 +353,8 @@ SHISO_API int shiso_causal_conv(const void* x, long long x_ld, int act_dtype, co
 // (2i, 2i + 1) - turned by positions[t] * inv_freq[i], cosine and sine times `magnitude`; columns
 // from rotary_dim on are copied.  x and out are [T, H, width] with their own row and head strides.
 template <typename AT>
-__global__ void rotate_heads_kernel(const AT* __restrict__ x, long long x_ld, long long x_hs, AT* __restrict__ out, long long out_ld,
-                                    long long out_hs, const float* __restrict__ inv_freq, const int* __restrict__ positions,
+__global__ void rotate_heads_kernel(const AT* x, long long x_ld, long long x_hs, AT* __restrict__ out, long long out_ld,
+                                    long long out_hs, const float* __restrict__ inv_freq, const int* positions,
                                     int tokens, int heads, int width, int rotary_dim, float magnitude, int interleaved) {
     pdl_begin();
     const int half = rotary_dim / 2;
@@ -403,9 +403,9 @@ SHISO_API int shiso_rotate_heads(const void* x, long long x_ld, long long x_hs, 
 // square, times w; the rest rotated by the position (pairs and magnitude as in rotate_heads_kernel);
 // both stored as the position's cache row.  One block per row.
 template <typename AT>
-__global__ void latent_store_kernel(const AT* __restrict__ rows, long long ld, const float* __restrict__ w,
-                                    const float* __restrict__ inv_freq, const int* __restrict__ positions,
-                                    const int* __restrict__ seq_of_token, const int* __restrict__ block_table, int table_width,
+__global__ void latent_store_kernel(const AT* rows, long long ld, const float* __restrict__ w,
+                                    const float* __restrict__ inv_freq, const int* positions,
+                                    const int* seq_of_token, const int* block_table, int table_width,
                                     AT* __restrict__ cache, int rank, int width, int rotary_dim, int page_size, float eps,
                                     float magnitude, int interleaved) {
     pdl_begin();

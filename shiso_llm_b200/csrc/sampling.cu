@@ -67,7 +67,7 @@ __device__ __forceinline__ void hand_over_status(int* status_word, int* status_o
         *status_out = atomicExch(status_word, 0);
 }
 
-__global__ void suppress_kernel(float* __restrict__ logits, const int* __restrict__ rows, const int* __restrict__ ids,
+__global__ void suppress_kernel(float* logits, const int* rows, const int* ids,
                                 int count, int num_rows, int vocab) {
     pdl_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -76,7 +76,7 @@ __global__ void suppress_kernel(float* __restrict__ logits, const int* __restric
     if (r >= 0 && r < num_rows && id >= 0 && id < vocab) logits[(size_t)r * vocab + id] = -INFINITY;
 }
 
-__global__ void __launch_bounds__(THREADS) argmax_kernel(const float* __restrict__ logits, int* __restrict__ out, int vocab,
+__global__ void __launch_bounds__(THREADS) argmax_kernel(const float* logits, int* __restrict__ out, int vocab,
                                                          int* status_word, int* status_out) {
     pdl_begin();
     hand_over_status(status_word, status_out);
@@ -95,7 +95,7 @@ __global__ void __launch_bounds__(THREADS) argmax_kernel(const float* __restrict
 // so that a handful of rows still keeps many SMs reading; the second stage picks among the
 // chunk winners (ascending chunk order, so the lower id still wins a tie).
 __global__ void __launch_bounds__(256)
-argmax_chunk_kernel(const float* __restrict__ logits, float* __restrict__ best_v, int* __restrict__ best_i, int vocab,
+argmax_chunk_kernel(const float* logits, float* __restrict__ best_v, int* __restrict__ best_i, int vocab,
                     int chunk_len, int chunks) {
     pdl_begin();
     __shared__ Best scratch[32];
@@ -125,7 +125,7 @@ argmax_chunk_kernel(const float* __restrict__ logits, float* __restrict__ best_v
     }
 }
 
-__global__ void argmax_final_kernel(const float* __restrict__ best_v, const int* __restrict__ best_i,
+__global__ void argmax_final_kernel(const float* best_v, const int* best_i,
                                     int* __restrict__ out, int chunks, int* status_word, int* status_out) {
     pdl_begin();
     hand_over_status(status_word, status_out);
@@ -178,7 +178,7 @@ __device__ __forceinline__ unsigned long long fixed_mass(float scaled /* (l - ma
 // 8-bit radix passes; weight is 1 (count, for top-k) or the fixed-point mass (top-p).
 // Only entries with key >= floor_key take part.  All threads return the same K.
 template <bool MASS>
-__device__ unsigned radix_threshold(const float* __restrict__ row, int vocab, float max_logit, float inv_t,
+__device__ unsigned radix_threshold(const float* row, int vocab, float max_logit, float inv_t,
                                     unsigned floor_key, unsigned long long target,
                                     unsigned long long* hist /* 256 */, unsigned* shared_u /* 2 */) {
     unsigned prefix = 0, prefix_mask = 0;
@@ -221,9 +221,9 @@ __device__ unsigned radix_threshold(const float* __restrict__ row, int vocab, fl
 }
 
 __global__ void __launch_bounds__(THREADS)
-sample_kernel(const float* __restrict__ logits, const float* __restrict__ temperature, const int* __restrict__ top_k,
-              const float* __restrict__ top_p, const float* __restrict__ min_p,
-              const long long* __restrict__ keys, const int* __restrict__ positions, int* __restrict__ out, int vocab,
+sample_kernel(const float* logits, const float* temperature, const int* top_k,
+              const float* top_p, const float* min_p,
+              const long long* keys, const int* positions, int* __restrict__ out, int vocab,
               int* status_word, int* status_out) {
     pdl_begin();
     hand_over_status(status_word, status_out);
@@ -292,7 +292,7 @@ sample_kernel(const float* __restrict__ logits, const float* __restrict__ temper
 // reads or writes in place: a step's few tokens reach the host (and its few KB of row data the
 // device) as loads and stores of a kernel in the stream, without a turn of the copy engine
 // between two kernels.
-__global__ void __launch_bounds__(256) copy_words_kernel(const int* __restrict__ src, int* __restrict__ dst, int n) {
+__global__ void __launch_bounds__(256) copy_words_kernel(const int* src, int* __restrict__ dst, int n) {
     pdl_begin();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) dst[i] = src[i];
 }

@@ -20,7 +20,7 @@ constexpr int MAX_TAPS = 8;
 // u at relative time `rel` of a sequence whose rows start at `first`: from this step's
 // rows when rel >= 0, else from the state (index taps-1+rel).
 template <typename AT>
-__device__ __forceinline__ float gated_input(const AT* __restrict__ proj, const float* __restrict__ state_row,
+__device__ __forceinline__ float gated_input(const AT* proj, const float* state_row,
                                              int first, int rel, int ch, int hidden, int taps, long long state_stride_t) {
     if (rel >= 0) {
         const AT* row = proj + (size_t)(first + rel) * 3 * hidden;
@@ -30,10 +30,10 @@ __device__ __forceinline__ float gated_input(const AT* __restrict__ proj, const 
 }
 
 template <typename AT>
-__global__ void short_conv_out_kernel(const AT* __restrict__ proj, const float* __restrict__ w,
-                                      const float* __restrict__ bias, const float* __restrict__ state,
-                                      long long slot_stride, const int* __restrict__ seq_of_token,
-                                      const int* __restrict__ q_start, const int* __restrict__ slots,
+__global__ void short_conv_out_kernel(const AT* proj, const float* __restrict__ w,
+                                      const float* __restrict__ bias, const float* state,
+                                      long long slot_stride, const int* seq_of_token,
+                                      const int* q_start, const int* slots,
                                       AT* __restrict__ y, int hidden, int taps) {
     pdl_begin();
     const int t = blockIdx.x;
@@ -136,8 +136,8 @@ __device__ __forceinline__ void gated8(const uint4& braw, const uint4& xraw, flo
 template <int TAPS, int RUN>
 __global__ void __launch_bounds__(128)
 short_conv_run_kernel(const __nv_bfloat16* proj, const float* __restrict__ w, const float* __restrict__ bias,
-                      const float* state, long long slot_stride, const int* __restrict__ seq_of_token,
-                      const int* __restrict__ q_start, const int* __restrict__ slots, __nv_bfloat16* y,
+                      const float* state, long long slot_stride, const int* seq_of_token,
+                      const int* q_start, const int* slots, __nv_bfloat16* y,
                       int hidden, int tokens) {
     pdl_begin();
     const int ch = (blockIdx.y * blockDim.x + threadIdx.x) * 8;
@@ -267,9 +267,9 @@ short_conv_run_kernel(const __nv_bfloat16* proj, const float* __restrict__ w, co
 // New state = the last taps-1 values of (old state ++ this step's u).  One thread owns a
 // (sequence, channel) pair and reads everything it needs before it writes.
 template <typename AT>
-__global__ void short_conv_state_kernel(const AT* __restrict__ proj, float* __restrict__ state,
-                                        long long slot_stride, const int* __restrict__ q_start,
-                                        const int* __restrict__ slots, int hidden, int taps) {
+__global__ void short_conv_state_kernel(const AT* proj, float* state,
+                                        long long slot_stride, const int* q_start,
+                                        const int* slots, int hidden, int taps) {
     pdl_begin();
     const int s = blockIdx.x;
     const int ch = blockIdx.y * blockDim.x + threadIdx.x;
@@ -296,10 +296,10 @@ __global__ void short_conv_state_kernel(const AT* __restrict__ proj, float* __re
 // (kernels/metal/dense/dense_short_conv.metal:45-67).  Nothing else touches that pair's
 // state, so reading and rewriting it in one kernel is safe.
 template <typename AT>
-__global__ void short_conv_serial_kernel(const AT* __restrict__ proj, const float* __restrict__ w,
-                                         const float* __restrict__ bias, float* __restrict__ state,
-                                         long long slot_stride, const int* __restrict__ q_start,
-                                         const int* __restrict__ slots, AT* __restrict__ y, int hidden, int taps) {
+__global__ void short_conv_serial_kernel(const AT* proj, const float* __restrict__ w,
+                                         const float* __restrict__ bias, float* state,
+                                         long long slot_stride, const int* q_start,
+                                         const int* slots, AT* __restrict__ y, int hidden, int taps) {
     pdl_begin();
     const int s = blockIdx.x;
     const int ch = blockIdx.y * blockDim.x + threadIdx.x;

@@ -24,10 +24,10 @@ __device__ __forceinline__ int step_token(const int* ids, const int* feed_index,
 // slot holds (token + 1).  The slots are written by the kernel below, after this one.  A step's first
 // kernel, launched in full order: common.cuh says why.
 template <typename WT>
-__global__ void embed_hashed_pair_kernel(const int* __restrict__ ids, const int* __restrict__ feed_index, const int* fed_tokens,
+__global__ void embed_hashed_pair_kernel(const int* ids, const int* feed_index, const int* fed_tokens,
                                          const WT* __restrict__ table, const WT* __restrict__ pair_table,
-                                         const int* __restrict__ seq_of_token, const int* __restrict__ q_start,
-                                         const int* __restrict__ start_pos, const int* __restrict__ slots,
+                                         const int* seq_of_token, const int* q_start,
+                                         const int* start_pos, const int* slots,
                                          const int* state, long long state_stride, float* __restrict__ out,
                                          int hidden, int vocab, float scale, int buckets, int mul_prev, int mul_cur) {
     pdl_begin();
@@ -46,8 +46,8 @@ __global__ void embed_hashed_pair_kernel(const int* __restrict__ ids, const int*
     for (int i = threadIdx.x; i < hidden; i += blockDim.x) dst[i] = valid ? to_f32(e[i]) * scale + to_f32(b[i]) : 0.0f;
 }
 
-__global__ void store_last_token_kernel(const int* __restrict__ ids, const int* __restrict__ feed_index, const int* fed_tokens,
-                                        const int* __restrict__ q_start, const int* __restrict__ slots, int* state,
+__global__ void store_last_token_kernel(const int* ids, const int* feed_index, const int* fed_tokens,
+                                        const int* q_start, const int* slots, int* state,
                                         long long state_stride, int num_seqs) {
     pdl_begin();
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -88,7 +88,7 @@ constexpr int MAX_COPIES = 8;
 // u * rsqrt(mean(u^2) + eps) * norm_w, into `normed`.  With `sum_out`: sum_r x_r'.  `src` has
 // `copies` lanes `src_stride` floats apart (0: one stream stands for every copy).
 template <typename AT>
-__global__ void hyper_mix_kernel(const float* src, long long src_stride, const AT* __restrict__ y,
+__global__ void hyper_mix_kernel(const float* src, long long src_stride, const AT* y,
                                  const float* __restrict__ mix, const float* __restrict__ write, float* dst, long long dst_stride,
                                  const float* __restrict__ read, const float* __restrict__ norm_w, float eps,
                                  AT* __restrict__ normed, float* __restrict__ sum_out, int hidden, int copies) {
@@ -337,10 +337,10 @@ SHISO_API int shiso_hyper_mix(const float* src, long long src_stride, const void
 // out[c, t, :] = h_t + (h_{t-1} - h_t) * mu[c, :] for c < blends, with h_{t-1} the row before in
 // the same sequence, the request's stored row for a portion's first token, zeros at position 0.
 template <typename AT>
-__global__ void token_shift_blend_kernel(const AT* __restrict__ h, const float* __restrict__ mu, const float* state,
-                                         long long state_stride, const int* __restrict__ seq_of_token,
-                                         const int* __restrict__ q_start, const int* __restrict__ start_pos,
-                                         const int* __restrict__ slots, AT* __restrict__ out, int tokens, int hidden, int blends) {
+__global__ void token_shift_blend_kernel(const AT* h, const float* __restrict__ mu, const float* state,
+                                         long long state_stride, const int* seq_of_token,
+                                         const int* q_start, const int* start_pos,
+                                         const int* slots, AT* __restrict__ out, int tokens, int hidden, int blends) {
     pdl_begin();
     const int t = blockIdx.x;
     const int s = seq_of_token[t];
@@ -363,9 +363,9 @@ __global__ void token_shift_blend_kernel(const AT* __restrict__ h, const float* 
 constexpr int SHIFT_RUN = 4;
 template <typename AT>
 __global__ void __launch_bounds__(128) token_shift_blend_quads_kernel(const AT* h, const float* __restrict__ mu, const float* state,
-                                                                      long long state_stride, const int* __restrict__ seq_of_token,
-                                                                      const int* __restrict__ q_start, const int* __restrict__ start_pos,
-                                                                      const int* __restrict__ slots, AT* __restrict__ out, int tokens,
+                                                                      long long state_stride, const int* seq_of_token,
+                                                                      const int* q_start, const int* start_pos,
+                                                                      const int* slots, AT* __restrict__ out, int tokens,
                                                                       int hidden, int blends) {
     pdl_begin();
     const int i = (blockIdx.y * 128 + threadIdx.x) * 4;
@@ -400,8 +400,8 @@ __global__ void __launch_bounds__(128) token_shift_blend_quads_kernel(const AT* 
 }
 
 template <typename AT>
-__global__ void store_last_row_kernel(const AT* __restrict__ h, float* state, long long state_stride,
-                                      const int* __restrict__ q_start, const int* __restrict__ slots, int hidden) {
+__global__ void store_last_row_kernel(const AT* h, float* state, long long state_stride,
+                                      const int* q_start, const int* slots, int hidden) {
     pdl_begin();
     const int s = blockIdx.x;
     const int a = q_start[s], e = q_start[s + 1];
@@ -436,7 +436,7 @@ SHISO_API int shiso_token_shift_blend(const void* h, int act_dtype, const float*
 enum { SHISO_UNARY_TANH = 0, SHISO_UNARY_SILU = 1, SHISO_UNARY_RELU2 = 2, SHISO_UNARY_COPY = 3 };  // relu2: the square of max(x, 0); copy: the value in the output's type
 
 template <typename IT, typename OT>
-__global__ void unary_kernel(const IT* __restrict__ x, OT* __restrict__ out, long long count, int kind) {
+__global__ void unary_kernel(const IT* x, OT* __restrict__ out, long long count, int kind) {
     pdl_begin();
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (long long)gridDim.x * blockDim.x) {
         const float v = to_f32(x[i]);

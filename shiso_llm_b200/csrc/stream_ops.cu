@@ -96,7 +96,7 @@ template <int N> __device__ __forceinline__ void store_n(__nv_bfloat16* p, const
 // One thread per N neighbouring columns of a row.
 template <typename AT, int N>
 __global__ void __launch_bounds__(256)
-add_dyt_kernel(float* __restrict__ residual, const AT* __restrict__ d0, const AT* __restrict__ d1, const int* __restrict__ rows,
+add_dyt_kernel(float* residual, const AT* d0, const AT* d1, const int* rows,
                const float* __restrict__ w, const float* __restrict__ b, float alpha, AT* __restrict__ out, int out_rows, int hidden) {
     pdl_begin();
     const int per_row = hidden / N;
@@ -186,7 +186,7 @@ SHISO_API int shiso_stream_add(const float* residual, float* out, const void* d0
 // A thread per N neighbouring columns.
 template <typename AT, int N>
 __global__ void __launch_bounds__(256)
-stream_add_rows_kernel(float* __restrict__ residual, const AT* __restrict__ d0, const AT* __restrict__ d1, float scale,
+stream_add_rows_kernel(float* residual, const AT* d0, const AT* d1, float scale,
                        AT* __restrict__ rows, long long total) {
     pdl_begin();
     const long long i = ((long long)blockIdx.x * blockDim.x + threadIdx.x) * N;
@@ -229,8 +229,8 @@ SHISO_API int shiso_stream_add_rows(float* residual, const void* d0, const void*
 
 template <typename WT, typename AT>
 __global__ void __launch_bounds__(256)
-side_gate_kernel(const float* __restrict__ z, const WT* __restrict__ table, long long table_ld, int first_column, int vocab,
-                 const int* __restrict__ ids, const int* __restrict__ feed_index, const int* __restrict__ fed_tokens, AT* __restrict__ out,
+side_gate_kernel(const float* z, const WT* __restrict__ table, long long table_ld, int first_column, int vocab,
+                 const int* ids, const int* feed_index, const int* fed_tokens, AT* __restrict__ out,
                  int tokens, int dim) {
     pdl_begin();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -326,7 +326,7 @@ SHISO_API int shiso_stream_concat(const float* residual, const void* d0, int d0_
 
 template <typename AT>
 __global__ void __launch_bounds__(256)
-glu_act_kernel(const AT* __restrict__ gate_up, AT* __restrict__ out, int inter, long long total, int act, float limit) {
+glu_act_kernel(const AT* gate_up, AT* __restrict__ out, int inter, long long total, int act, float limit) {
     pdl_begin();
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= total) return;
@@ -357,7 +357,7 @@ SHISO_API int shiso_glu_act(const void* gate_up, void* out, int act_dtype, int t
 // x[t, c] *= sigmoid(gate[t, c]) in place; rows of x and of the gate have their own strides.
 template <typename AT, int N>
 __global__ void __launch_bounds__(256)
-gate_rows_kernel(AT* __restrict__ x, long long x_ld, const AT* __restrict__ gate, long long gate_ld, int tokens, int cols) {
+gate_rows_kernel(AT* x, long long x_ld, const AT* gate, long long gate_ld, int tokens, int cols) {
     pdl_begin();
     const int per_row = cols / N;
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -444,9 +444,9 @@ __device__ __forceinline__ void norm_rotate_columns(const AT* src, AT* dst, cons
 // and every pointer 16-byte aligned); the order of a row's sums depends on the block's size only.
 template <typename AT, int N>
 __global__ void __launch_bounds__(256)
-joined_norm_store_kernel(AT* __restrict__ proj, long long ld, int q_cols, int k_cols, int v_col, int v_cols, const float* __restrict__ q_w,
-                         const float* __restrict__ k_w, const int* __restrict__ positions, const int* __restrict__ seq_of_token,
-                         const int* __restrict__ table, int table_width, AT* __restrict__ k_cache, AT* __restrict__ v_cache,
+joined_norm_store_kernel(AT* proj, long long ld, int q_cols, int k_cols, int v_col, int v_cols, const float* __restrict__ q_w,
+                         const float* __restrict__ k_w, const int* positions, const int* seq_of_token,
+                         const int* table, int table_width, AT* __restrict__ k_cache, AT* __restrict__ v_cache,
                          int page_size, float eps, float temp_coef, int temp_every, const Rotation rot) {
     pdl_begin();
     __shared__ float scratch[33];

@@ -8,6 +8,28 @@ from shiso_llm_b200.kernels import build
 
 SOURCES = {os.path.basename(p): open(p, encoding="utf-8").read() for p in build.sources()}
 
+# Pointers that may be __restrict__ const: weights and other tensors that no kernel writes.
+WEIGHTS = {"q_w", "k_w", "inv_freq", "w", "bias", "b", "pair_table", "coefficients", "norm_w", "taps", "mu", "correction", "mix", "write", "read"}
+
+
+def kernels(text):
+    """(name, parameters) of every kernel of a file."""
+    pattern = re.compile(r"__global__\s+void\s*(?:__launch_bounds__\((?:[^()]|\([^()]*\))*\)\s*)?(\w+)\s*\(([^{]*?)\)\s*\{")
+    return [(m.group(1), re.sub(r"\s+", " ", m.group(2))) for m in pattern.finditer(text)]
+
+
+def test_nothing_a_kernel_writes_is_read_through_restrict_const():
+    found = []
+    for name, text in SOURCES.items():
+        for kernel, parameters in kernels(text):
+            for kind, what in re.findall(r"const ([\w ]+)\* __restrict__ (\w+)", parameters):
+                if what not in WEIGHTS and not (what == "table" and kind == "WT"):
+                    found.append((name, kernel, what))
+            # read and written in place
+            found += [(name, kernel, what) for what in re.findall(r"(?<!const )\b\w+\* __restrict__ (residual|proj|logits|state|x)\b", parameters)
+                      if not re.search(r"const [\w ]+\* __restrict__ " + what, parameters)]
+    assert sum(len(kernels(t)) for t in SOURCES.values()) > 60 and not found, found
+
 
 def test_a_steps_first_kernel_is_launched_in_full_order():
     """What uploads a step's data lets its successor start early, and kernels read step data ahead of their wait."""
