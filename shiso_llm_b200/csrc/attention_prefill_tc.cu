@@ -32,8 +32,9 @@
 // are masked in the scores and zeroed in the value tile before the second product, so nothing
 // stored there can reach the result.
 //
-// Every mbarrier wait is bounded; a wait that runs out sets the status word and the kernel carries
-// on to its end (TMEM is freed), its result then being wrong.
+// Every mbarrier wait is bounded, and each role leaves its loop at the first wait that runs out: the roles wait
+// for one another at the same time, so a signal that is lost costs a CTA one limit and not one a tile.  The
+// copies and products still in flight are waited for (with the same limit), TMEM is freed, the status word is set, and the result is wrong.
 #include "tcgen05.cuh"
 
 namespace {
@@ -138,7 +139,8 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     uint64_t* s_full = v_empty + STAGES;      // [2] the scores of a tile are complete
     uint64_t* p_full = s_full + 2;            // [2] its P is written (and its scores are read)
     uint64_t* pv_done = p_full + 2;           // [2] its product with the values is complete
-    uint32_t* tmem_slot = (uint32_t*)(pv_done + 2);
+    uint64_t* products_done = pv_done + 2;    // nothing of this CTA is left in the tensor core
+    uint32_t* tmem_slot = (uint32_t*)(products_done + 1);
     int* shared_ints = (int*)(tmem_slot + 1);  // [0] failed, [1] sequence, [2] first row of the tile
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -158,6 +160,11 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             mbar_init(&p_full[i], 4);  // one arrival per softmax warp
             mbar_init(&pv_done[i], 1);
         }
+        mbar_init(products_done, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (threadIdx.x == 0) {
         shared_ints[0] = 0;
         // which (sequence, tile) is this CTA?  The last tiles of a portion have the most keys:
         // they take the first CTAs - of every head, the head being the grid's fast index - so
@@ -176,8 +183,6 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         }
         shared_ints[1] = found;
         shared_ints[2] = row0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     __syncthreads();
     const int seq = shared_ints[1];
@@ -224,7 +229,8 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             return page >= 0 ? page * a.page_size : a.cache_rows;  // a row past the end of the cache: zeros
         };
         int row_next = lookup(0);
-        for (int it = 0; it < num_tiles; ++it) {
+        int asked = 0;  // copies of tiles begun: keys and values in turn
+        for (int it = 0; it < num_tiles && !failed; ++it) {
             const int s = it % STAGES, uses_before = it / STAGES;
             const int row = row_next;
             if (it + 1 < num_tiles) row_next = lookup(it + 1);
@@ -232,12 +238,21 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                 uint64_t* full = kv ? &v_full[s] : &k_full[s];
                 uint64_t* empty = kv ? &v_empty[s] : &k_empty[s];
                 uint8_t* dst = (kv ? v_s : k_s) + s * KV_BYTES;
-                if (uses_before > 0 && !mbar_wait(empty, (uses_before - 1) & 1)) failed = true;
+                if (uses_before > 0 && !__all_sync(0xffffffffu, mbar_wait(empty, (uses_before - 1) & 1))) {
+                    failed = true;
+                    break;
+                }
                 if (lane == 0) mbar_expect_tx(full, KV_BYTES);
                 __syncwarp();
                 if (lane < pages_per_tile) tma_load_3d(dst + lane * a.page_size * ROW, kv ? &map_v : &map_k, 0, kv_head, row, full);
+                ++asked;
             }
         }
+        // the shared memory is not given back before the last copies into it have landed
+        bool landed = mbar_wait(q_full, 0);
+        for (int i = max(0, asked - 2 * STAGES); i < asked && landed; ++i)
+            landed = mbar_wait((i & 1) ? &v_full[(i >> 1) % STAGES] : &k_full[(i >> 1) % STAGES], ((i >> 1) / STAGES) & 1);
+        if (!landed) failed = true;
     } else if (warp == 5) {
         // ---- MMA issuer
         if (lane == 0) {
@@ -247,7 +262,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             const uint32_t q_addr = smem_u32(q_s);
             auto scores = [&](int it) {
                 const int s = it % STAGES;
-                if (!mbar_wait(&k_full[s], (it / STAGES) & 1)) failed = true;
+                if (!mbar_wait(&k_full[s], (it / STAGES) & 1)) return false;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t k_addr = smem_u32(k_s + s * KV_BYTES);
 #pragma unroll
@@ -255,16 +270,17 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                     umma_bf16(tmem_base + S_COL + (it & 1) * BKEY, umma_desc(q_addr + ks * 32), umma_desc(k_addr + ks * 32), idesc_s, ks > 0 ? 1u : 0u);
                 umma_commit(&s_full[it & 1]);
                 umma_commit(&k_empty[s]);
+                return true;
             };
-            if (!mbar_wait(q_full, 0)) failed = true;
-            scores(0);
-            if (num_tiles > 1) scores(1);
-            for (int it = 0; it < num_tiles; ++it) {
+            if (!mbar_wait(q_full, 0) || !scores(0) || (num_tiles > 1 && !scores(1))) failed = true;
+            for (int it = 0; it < num_tiles && !failed; ++it) {
                 const int b = it & 1, vs = it % STAGES;
-                if (!mbar_wait(&p_full[b], (it >> 1) & 1)) failed = true;   // P is written, its scores are read
+                failed = !mbar_wait(&p_full[b], (it >> 1) & 1);  // P is written, its scores are read
+                if (failed) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (it + 2 < num_tiles) scores(it + 2);  // into the buffer this tile's scores left
-                if (!mbar_wait(&v_full[vs], (it / STAGES) & 1)) failed = true;
+                failed = (it + 2 < num_tiles && !scores(it + 2))  // into the buffer this tile's scores left
+                         || !mbar_wait(&v_full[vs], (it / STAGES) & 1);
+                if (failed) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t v_addr = smem_u32(v_s + vs * KV_BYTES);
 #pragma unroll
@@ -274,6 +290,8 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
                 umma_commit(&pv_done[b]);
                 umma_commit(&v_empty[vs]);
             }
+            umma_commit(products_done);
+            if (!mbar_wait(products_done, 0)) failed = true;
         }
     } else {
         // ---- softmax warps: thread = (token, query head) = TMEM lane
@@ -282,12 +300,14 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         const int my_pos = first_pos + my_token;
         const uint32_t lane_base = tmem_base + ((uint32_t)(warp * 32) << 16);
         float row_max = -INFINITY, row_sum = 0.0f;  // the maximum in use (scaled, log2 units) and the sum against it
+        auto wait = [&](uint64_t* bar, int use) { return __all_sync(0xffffffffu, mbar_wait(bar, use & 1)); };  // the warp leaves together
         for (int it = 0; it < num_tiles; ++it) {
             const int b = it & 1;
             const int key0 = tile_at(it) * BKEY;
             // every key of the tile is seen by every row of the CTA: no mask, nothing to zero
             const bool open = it >= kept_tiles && key0 + BKEY - 1 <= first_pos && (a.window <= 0 || key0 > first_pos + per_tile - 1 - a.window);
-            if (!mbar_wait(&s_full[b], (it >> 1) & 1)) failed = true;
+            failed = !wait(&s_full[b], it >> 1);
+            if (failed) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             uint32_t sv[BKEY];
             tmem_ld32_issue(lane_base + S_COL + b * BKEY, sv);
@@ -316,11 +336,13 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             const float base = new_max == -INFINITY ? 0.0f : new_max;  // a row that has seen nothing yet
             const float alpha = ex2(row_max - base);                   // exp2(-inf) = 0 for a first maximum, 1 when unchanged
             // this tile's P buffer was the A operand of the product two tiles back
-            if (it >= 2 && !mbar_wait(&pv_done[b], ((it - 2) >> 1) & 1)) failed = true;
+            failed = it >= 2 && !wait(&pv_done[b], (it - 2) >> 1);
+            if (failed) break;
             if (it > 0 && __any_sync(0xffffffffu, new_max != row_max)) {
                 // some row of this warp raises its maximum: every product issued so far must be
                 // complete, then O *= exp2(old - new) in tensor memory
-                if (!mbar_wait(&pv_done[b ^ 1], ((it - 1) >> 1) & 1)) failed = true;
+                failed = !wait(&pv_done[b ^ 1], (it - 1) >> 1);
+                if (failed) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 uint32_t o[32];
 #pragma unroll 1
@@ -359,7 +381,8 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             if (!open) {
                 // thread r also looks after value row r of the tile: outside the range it becomes zero
                 const int vs = it % STAGES;
-                if (!mbar_wait(&v_full[vs], (it / STAGES) & 1)) failed = true;
+                failed = !wait(&v_full[vs], it / STAGES);
+                if (failed) break;
                 const int key = key0 + r;
                 if (r < BKEY && ((key < key_lo && key >= a.keep_first) || key > last_pos)) {
                     uint4* row = reinterpret_cast<uint4*>(v_s + vs * KV_BYTES + r * ROW);
@@ -374,7 +397,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
             if (lane == 0) mbar_arrive(&p_full[b]);
         }
         pdl_trigger();
-        if (!mbar_wait(&pv_done[(num_tiles - 1) & 1], ((num_tiles - 1) >> 1) & 1)) failed = true;
+        if (!failed) failed = !wait(&pv_done[(num_tiles - 1) & 1], (num_tiles - 1) >> 1);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         // (a sink that outweighs every key by 2^128 makes its share infinite and the output the zero it tends to)
         if (a.sink && row_sum > 0.0f) row_sum += exp2f(a.sink[head] * 1.4426950408889634f - row_max);

@@ -22,8 +22,8 @@
 // Key and value tiles come from the paged cache by TMA, one box per page and 64 channels, four stages
 // ahead.  The cache's rows of a key head are [map 1 | map 2]: two boxes where D = 64, one where D = 32.
 // Pages outside the rows' range are fetched past the end of the cache (zeros); rows outside it are
-// masked in the scores and zeroed in the value tile.  512 tensor-memory columns, one CTA an SM.  Every
-// mbarrier wait is bounded and reports through the status word.
+// masked in the scores and zeroed in the value tile.  512 tensor-memory columns, one CTA an SM.  Every mbarrier wait is bounded; each role leaves its loop at the first that runs out, and
+// the status word says so (see attention_prefill_tc.cu).
 #include "tcgen05.cuh"
 
 namespace {
@@ -121,7 +121,8 @@ differential_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     uint64_t* s_free = s_full + 2;                 // [map] they are in registers
     uint64_t* p_full = s_free + 2;                 // [map][2] a tile's P is written
     uint64_t* pv_done = p_full + 4;                // [map][2] its product with the values is complete
-    uint32_t* tmem_slot = (uint32_t*)(pv_done + 4);
+    uint64_t* products_done = pv_done + 4;         // nothing of this CTA is left in the tensor core
+    uint32_t* tmem_slot = (uint32_t*)(products_done + 1);
     int* shared_ints = (int*)(tmem_slot + 1);      // failed, sequence, first row of the tile
     float* row_inv = (float*)((uint8_t*)bars + 512);  // [map][BQ]
     float* row_ss = row_inv + 2 * BQ;                 // [half][BQ]
@@ -143,6 +144,11 @@ differential_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             mbar_init(&p_full[i], 4);
             mbar_init(&pv_done[i], 1);
         }
+        mbar_init(products_done, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    }
+    if (threadIdx.x == 0) {
         shared_ints[0] = 0;
         // the last tiles of a portion have the most keys: they take the first CTAs of every head
         int left = gridDim.y - 1 - blockIdx.y, found = -1, row0 = 0;
@@ -157,8 +163,6 @@ differential_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         }
         shared_ints[1] = found;
         shared_ints[2] = row0;
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
     __syncthreads();
     const int seq = shared_ints[1];
@@ -199,22 +203,32 @@ differential_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             return page >= 0 ? page * a.page_size : a.cache_rows;  // a row past the end of the cache: zeros
         };
         int row_next = lookup(0);
+        int asked = 0;  // copies of tiles begun: keys and values in turn
         for (int it = 0; it < num_tiles; ++it) {
             const int s = it % STAGES, uses_before = it / STAGES, row = row_next;
             if (it + 1 < num_tiles) row_next = lookup(it + 1);
-            if (uses_before > 0 && !mbar_wait(&k_empty[s], (uses_before - 1) & 1)) failed = true;
+            failed = uses_before > 0 && !__all_sync(0xffffffffu, mbar_wait(&k_empty[s], (uses_before - 1) & 1));
+            if (failed) break;
             if (lane == 0) mbar_expect_tx(&k_full[s], L::K_BYTES);
             __syncwarp();
             if (lane < pages_per_tile)
                 for (int b = 0; b < L::KB; ++b)
                     tma_load_3d(k_s + s * L::K_BYTES + b * TILE_BYTES + lane * a.page_size * ROW, &map_k, 0, kv_head * L::KB + b, row, &k_full[s]);
-            if (uses_before > 0 && !mbar_wait(&v_empty[s], (uses_before - 1) & 1)) failed = true;
+            ++asked;
+            failed = uses_before > 0 && !__all_sync(0xffffffffu, mbar_wait(&v_empty[s], (uses_before - 1) & 1));
+            if (failed) break;
             if (lane == 0) mbar_expect_tx(&v_full[s], L::V_BYTES);
             __syncwarp();
             if (lane < pages_per_tile)
                 for (int b = 0; b < VH; ++b)
                     tma_load_3d(v_s + s * L::V_BYTES + b * TILE_BYTES + lane * a.page_size * ROW, &map_v, 0, kv_head * VH + b, row, &v_full[s]);
+            ++asked;
         }
+        // the shared memory is not given back before the last copies into it have landed
+        bool landed = mbar_wait(q_full, 0);
+        for (int i = max(0, asked - 2 * STAGES); i < asked && landed; ++i)
+            landed = mbar_wait((i & 1) ? &v_full[(i >> 1) % STAGES] : &k_full[(i >> 1) % STAGES], ((i >> 1) / STAGES) & 1);
+        if (!landed) failed = true;
     } else if (warp == 9) {
         // ---- MMA issuer
         if (lane == 0) {
@@ -222,7 +236,7 @@ differential_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             const uint32_t idesc_o = umma_idesc(BQ, 64) | (1u << 16);  // B (the value tile) is MN-major
             auto scores = [&](int m, int it) {
                 const int s = it % STAGES;
-                if (!mbar_wait(&k_full[s], (it / STAGES) & 1)) failed = true;
+                if (!mbar_wait(&k_full[s], (it / STAGES) & 1)) return false;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t q_addr = smem_u32(q_s + m * Q_BYTES);
                 const uint32_t k_addr = smem_u32(k_s + s * L::K_BYTES) + (D == 64 ? m * TILE_BYTES : m * D * 2);
@@ -231,21 +245,20 @@ differential_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                     umma_bf16(tmem_base + L::S_COL + m * BKEY, umma_desc(q_addr + ks * 32), umma_desc(k_addr + ks * 32), idesc_s, ks > 0 ? 1u : 0u);
                 umma_commit(&s_full[m]);
                 if (m == 1) umma_commit(&k_empty[s]);
+                return true;
             };
-            if (!mbar_wait(q_full, 0)) failed = true;
-            scores(0, 0);
-            scores(1, 0);
-            for (int it = 0; it < num_tiles; ++it) {
+            failed = !mbar_wait(q_full, 0) || !scores(0, 0) || !scores(1, 0);
+            for (int it = 0; it < num_tiles && !failed; ++it) {
                 const int b = it & 1, s = it % STAGES;
                 if (it + 1 < num_tiles)
-                    for (int m = 0; m < 2; ++m) {  // the next tile's scores, while this tile's exponentials are taken
-                        if (!mbar_wait(&s_free[m], it & 1)) failed = true;
+                    for (int m = 0; m < 2 && !failed; ++m) {  // the next tile's scores, while this tile's exponentials are taken
+                        failed = !mbar_wait(&s_free[m], it & 1);
                         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                        scores(m, it + 1);
+                        if (!failed) failed = !scores(m, it + 1);
                     }
-                for (int m = 0; m < 2; ++m) {
-                    if (!mbar_wait(&p_full[2 * m + b], (it >> 1) & 1)) failed = true;
-                    if (!mbar_wait(&v_full[s], (it / STAGES) & 1)) failed = true;
+                for (int m = 0; m < 2 && !failed; ++m) {
+                    failed = !mbar_wait(&p_full[2 * m + b], (it >> 1) & 1) || !mbar_wait(&v_full[s], (it / STAGES) & 1);
+                    if (failed) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 #pragma unroll
                     for (int h = 0; h < VH; ++h) {
@@ -259,6 +272,8 @@ differential_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 }
                 umma_commit(&v_empty[s]);
             }
+            umma_commit(products_done);
+            if (!mbar_wait(products_done, 0)) failed = true;
         }
     } else {
         // ---- softmax warps: thread = query row = TMEM lane, of map `m`
@@ -268,12 +283,14 @@ differential_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         const uint32_t lane_base = tmem_base + ((uint32_t)(quad * 32) << 16);
         const uint32_t s_tmem = lane_base + L::S_COL + m * BKEY, o_tmem = lane_base + L::O_COL + m * L::V;
         float row_max = -INFINITY, row_sum = 0.0f;  // the maximum in use (scaled, log2 units) and the sum against it
+        auto wait = [&](uint64_t* bar, int use) { return __all_sync(0xffffffffu, mbar_wait(bar, use & 1)); };  // the warp leaves together
         for (int it = 0; it < num_tiles; ++it) {
             const int b = it & 1;
             const int key0 = (tile_first + it) * BKEY;
             // every key of the tile is seen by every row of the CTA: no mask, nothing to zero
             const bool open = key0 + BKEY - 1 <= first_pos && (a.window <= 0 || key0 > first_pos + BQ - 1 - a.window);
-            if (!mbar_wait(&s_full[m], it & 1)) failed = true;
+            failed = !wait(&s_full[m], it);
+            if (failed) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             uint32_t sv[BKEY];
             tmem_ld32_issue(s_tmem, sv);
@@ -303,11 +320,13 @@ differential_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
             const float base = new_max == -INFINITY ? 0.0f : new_max;  // a row that has seen nothing yet
             const float alpha = ex2(row_max - base);
             // this tile's P buffer was the A operand of the product two tiles back
-            if (it >= 2 && !mbar_wait(&pv_done[2 * m + b], ((it - 2) >> 1) & 1)) failed = true;
+            failed = it >= 2 && !wait(&pv_done[2 * m + b], (it - 2) >> 1);
+            if (failed) break;
             if (it > 0 && __any_sync(0xffffffffu, new_max != row_max)) {
                 // some row of this warp raises its maximum: every product of this map issued so far must
                 // be complete, then O *= exp2(old - new) in tensor memory
-                if (!mbar_wait(&pv_done[2 * m + (b ^ 1)], ((it - 1) >> 1) & 1)) failed = true;
+                failed = !wait(&pv_done[2 * m + (b ^ 1)], (it - 1) >> 1);
+                if (failed) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 uint32_t o[32];
 #pragma unroll 1
@@ -345,7 +364,8 @@ differential_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
                 // map 1's thread r also looks after value row r of the tile (both maps' products wait for
                 // map 1's P): outside the range it becomes zero
                 const int vs = it % STAGES;
-                if (!mbar_wait(&v_full[vs], (it / STAGES) & 1)) failed = true;
+                failed = !wait(&v_full[vs], it / STAGES);
+                if (failed) break;
                 const int key = key0 + r;
                 if (r < BKEY && (key < key_lo || key > last_pos)) {
 #pragma unroll
@@ -366,7 +386,8 @@ differential_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         // ---- the difference: this map's warps take the channels [m * V / 2, (m + 1) * V / 2) of their rows
         constexpr int HALF = L::V / 2;
         // (each map's warps wait for their own last product: only they have followed that barrier's phases)
-        if (!mbar_wait(&pv_done[2 * m + ((num_tiles - 1) & 1)], ((num_tiles - 1) >> 1) & 1)) failed = true;
+        // (a warp that has left its loop goes on to here all the same: the others meet it below)
+        if (!failed) failed = !wait(&pv_done[2 * m + ((num_tiles - 1) & 1)], (num_tiles - 1) >> 1);
         row_inv[m * BQ + r] = row_sum > 0.0f ? 1.0f / row_sum : 0.0f;  // an empty span yields zeros
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         softmax_sync();

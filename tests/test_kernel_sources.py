@@ -4,6 +4,8 @@ kernels overlap.  (common.cuh states them, where it explains dependent launches.
 import os
 import re
 
+import pytest
+
 from shiso_llm_b200.kernels import build
 
 SOURCES = {os.path.basename(p): open(p, encoding="utf-8").read() for p in build.sources()}
@@ -36,3 +38,16 @@ def test_a_steps_first_kernel_is_launched_in_full_order():
     for name, kernel in (("elementwise.cu", "embed_kernel"), ("stream_copies.cu", "embed_hashed_pair_kernel")):
         launches = re.findall(r"(launch_\w+)\(" + kernel + "<", SOURCES[name])
         assert launches == ["launch_in_order"] * 2, (name, launches)
+
+
+@pytest.mark.parametrize("name", ["attention_prefill_tc.cu", "differential_attention_tc.cu"])
+def test_attention_leaves_at_the_first_wait_that_runs_out(name):
+    """Every wait is the condition of a way out of its loop; only the last ones of a role just note that they failed."""
+    text = SOURCES[name]
+    text = text[text.index("__global__"):]
+    text = text[: text.index("\n}\n")]
+    carried_on = [line.strip() for line in text.splitlines() if re.search(r"mbar_wait\(.*\)\) failed = true;", line)]
+    assert [line for line in carried_on if "products_done" not in line and "q_full" not in line] == []
+    waits = len(re.findall(r"(?<!auto )\bwait\(&|mbar_wait\(", text))
+    ways_out = len(re.findall(r"if \(failed\) break;|return false;|&& landed;|&& !failed|if \(!failed\) failed|products_done, 0\)|q_full, 0\)|break;", text))
+    assert waits >= 10 and ways_out >= waits - 3, (waits, ways_out)
