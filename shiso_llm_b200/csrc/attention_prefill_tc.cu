@@ -35,6 +35,9 @@
 // Every mbarrier wait is bounded, and each role leaves its loop at the first wait that runs out: the roles wait
 // for one another at the same time, so a signal that is lost costs a CTA one limit and not one a tile.  The
 // copies and products still in flight are waited for (with the same limit), TMEM is freed, the status word is set, and the result is wrong.
+//
+// Tensor memory is taken behind the wait for the kernel before: no CTA holds it, or waits for it, while
+// another grid's CTAs still have work to do with theirs.
 #include "tcgen05.cuh"
 
 namespace {
@@ -164,6 +167,7 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
+    pdl_wait();  // queries, keys and values were written by the kernels before this one
     if (threadIdx.x == 0) {
         shared_ints[0] = 0;
         // which (sequence, tile) is this CTA?  The last tiles of a portion have the most keys:
@@ -210,8 +214,6 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     const int num_tiles = kept_tiles + tile_last - tile_first + 1;
     auto tile_at = [&](int it) { return it < kept_tiles ? it : tile_first - kept_tiles + it; };
     bool failed = false;
-
-    pdl_wait();  // queries, keys and values were written by the kernels before this one
 
     if (warp == 4) {
         // ---- producer: lane p brings page p of every tile (its key box and its value box), and

@@ -22,7 +22,8 @@
 // Key and value tiles come from the paged cache by TMA, one box per page and 64 channels, four stages
 // ahead.  The cache's rows of a key head are [map 1 | map 2]: two boxes where D = 64, one where D = 32.
 // Pages outside the rows' range are fetched past the end of the cache (zeros); rows outside it are
-// masked in the scores and zeroed in the value tile.  512 tensor-memory columns, one CTA an SM.  Every mbarrier wait is bounded; each role leaves its loop at the first that runs out, and
+// masked in the scores and zeroed in the value tile.  512 tensor-memory columns, one CTA an SM, taken behind the
+// wait for the kernel before.  Every mbarrier wait is bounded; each role leaves its loop at the first that runs out, and
 // the status word says so (see attention_prefill_tc.cu).
 #include "tcgen05.cuh"
 
@@ -148,6 +149,7 @@ differential_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
+    pdl_wait();  // queries, keys and values were written by the kernels before this one
     if (threadIdx.x == 0) {
         shared_ints[0] = 0;
         // the last tiles of a portion have the most keys: they take the first CTAs of every head
@@ -184,8 +186,6 @@ differential_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     const int key_lo = a.window > 0 ? max(0, first_pos + 1 - a.window) : 0;  // the smallest key any row sees
     const int tile_first = key_lo / BKEY, num_tiles = last_pos / BKEY - tile_first + 1;
     bool failed = false;
-
-    pdl_wait();  // queries, keys and values were written by the kernels before this one
 
     if (warp == 8) {
         // ---- producer: lane p brings page p of every tile, looked up a tile ahead

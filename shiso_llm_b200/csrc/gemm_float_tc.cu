@@ -118,7 +118,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_float_tc_kernel(const __grid_
     uint64_t* empty = full + STAGES;
     uint64_t* acc_full = empty + STAGES;  // [2]
     uint64_t* acc_empty = acc_full + 2;   // [2]
-    uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
+    uint64_t* products_done = acc_empty + 2;  // nothing of this CTA is left in the tensor core
+    uint32_t* tmem_slot = (uint32_t*)(products_done + 1);
     int* failed = (int*)(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -136,11 +137,45 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_float_tc_kernel(const __grid_
             mbar_init(&acc_full[i], 1);
             mbar_init(&acc_empty[i], ADDERS);
         }
+        mbar_init(products_done, 1);
         *failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == 0) {
+    // splitting warps: unit u of a chunk is columns 8 (u % 8) .. + 7 of row u / 8
+    typedef std::integral_constant<int, 0> Even;
+    typedef std::integral_constant<int, 1> Odd;
+    const int row0 = threadIdx.x >> 3, piece = threadIdx.x & 7;
+    const bool has_x = !PIECES && row0 < NT;
+    const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    float4 wr[2][W_UNITS][2], xr[2][2];  // [chunk parity]
+    auto load_w = [&](int c, auto parity) {
+        const int k = k_begin + c * 64 + piece * 8;
+#pragma unroll
+        for (int i = 0; i < W_UNITS; ++i) {
+            const int n = n0 + row0 + 32 * i;
+            const float* p = a.w + (size_t)n * a.K + k;
+            wr[parity][i][0] = n < a.N && k < k_end ? __ldg((const float4*)p) : zero;
+            wr[parity][i][1] = n < a.N && k + 4 < k_end ? __ldg((const float4*)p + 1) : zero;
+        }
+    };
+    auto load_x = [&](int c, auto parity) {
+        const int k = k_begin + c * 64 + piece * 8, t = t0 + row0;
+        const float* p = a.x + (size_t)t * a.K + k;
+        xr[parity][0] = has_x && t < a.T && k < k_end ? *(const float4*)p : zero;
+        xr[parity][1] = has_x && t < a.T && k + 4 < k_end ? *((const float4*)p + 1) : zero;
+    };
+    if (warp < SPLITTERS) {
+        load_w(0, Even());  // (weights are no predecessor's output)
+        if (chunks > 1) load_w(1, Odd());
+    }
+    pdl_wait();
+    if (warp < SPLITTERS && !PIECES) {
+        load_x(0, Even());
+        if (chunks > 1) load_x(1, Odd());
+    }
+    // (behind the wait: no CTA holds tensor memory, or waits for it, while another grid's CTAs still work with theirs)
+    if (warp == SPLITTERS) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -150,27 +185,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_float_tc_kernel(const __grid_
     const uint32_t tmem_base = *tmem_slot;
 
     if (warp < SPLITTERS) {
-        // ---- unit u of a chunk: columns 8 (u % 8) .. + 7 of row u / 8
-        const int row0 = threadIdx.x >> 3, piece = threadIdx.x & 7;
-        const bool has_x = !PIECES && row0 < NT;
-        const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        float4 wr[2][W_UNITS][2], xr[2][2];  // [chunk parity]
-        auto load_w = [&](int c, auto parity) {
-            const int k = k_begin + c * 64 + piece * 8;
-#pragma unroll
-            for (int i = 0; i < W_UNITS; ++i) {
-                const int n = n0 + row0 + 32 * i;
-                const float* p = a.w + (size_t)n * a.K + k;
-                wr[parity][i][0] = n < a.N && k < k_end ? __ldg((const float4*)p) : zero;
-                wr[parity][i][1] = n < a.N && k + 4 < k_end ? __ldg((const float4*)p + 1) : zero;
-            }
-        };
-        auto load_x = [&](int c, auto parity) {
-            const int k = k_begin + c * 64 + piece * 8, t = t0 + row0;
-            const float* p = a.x + (size_t)t * a.K + k;
-            xr[parity][0] = has_x && t < a.T && k < k_end ? *(const float4*)p : zero;
-            xr[parity][1] = has_x && t < a.T && k + 4 < k_end ? *((const float4*)p + 1) : zero;
-        };
         auto work = [&](int c, auto parity) {
             const int s = c % STAGES;
             if (c >= STAGES && !mbar_wait(&empty[s], ((c / STAGES) - 1) & 1)) *failed = 1;
@@ -200,20 +214,19 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_float_tc_kernel(const __grid_
             __syncwarp();
             if (lane == 0) mbar_arrive(&full[s]);
         };
-        typedef std::integral_constant<int, 0> Even;
-        typedef std::integral_constant<int, 1> Odd;
-        load_w(0, Even());  // (weights are no predecessor's output)
-        if (chunks > 1) load_w(1, Odd());
-        pdl_wait();
-        if (!PIECES) {
-            load_x(0, Even());
-            if (chunks > 1) load_x(1, Odd());
-        }
+        int worked = 0;
         for (int c = 0; c < chunks; c += 2) {
             if (__any_sync(0xffffffffu, *(volatile int*)failed)) break;  // (a wait ran out: no further one is begun)
             work(c, Even());
             if (c + 1 < chunks) work(c + 1, Odd());
+            worked = min(chunks, c + 2);
         }
+        if (PIECES && threadIdx.x == 0)  // the shared memory is not given back before the last copies into it have landed
+            for (int c = max(0, worked - STAGES); c < worked; ++c)
+                if (!mbar_wait(&full[c % STAGES], (c / STAGES) & 1)) {
+                    *failed = 1;
+                    break;
+                }
     } else {
         // ---- adders: row n of W, rows t .. t + COLS - 1 of X
         const uint32_t idesc = umma_idesc(TILE_N, NT);
@@ -238,7 +251,6 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_float_tc_kernel(const __grid_
         const int n = n0 + q * 32 + lane, t = t0 + half * COLS;
         const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + half * COLS;
         const bool live = n < a.N;
-        pdl_wait();
         float sum[COLS];
         bool fresh = true;  // the next chunk is a group's first
         for (int c = 0; c < chunks; ++c) {
@@ -293,13 +305,17 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_float_tc_kernel(const __grid_
             }
             fresh = true;
         }
+        if (threadIdx.x == SPLITTERS * 32) {
+            umma_commit(products_done);
+            if (!mbar_wait(products_done, 0)) *failed = 1;
+        }
     }
     pdl_trigger();
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (*failed != 0 && threadIdx.x == 0 && a.status) atomicExch(a.status, 1);
-    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
+    if (warp == SPLITTERS) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
 }
 
 // y = the groups' sums in their order (+ bias).

@@ -51,3 +51,10 @@ def test_attention_leaves_at_the_first_wait_that_runs_out(name):
     waits = len(re.findall(r"(?<!auto )\bwait\(&|mbar_wait\(", text))
     ways_out = len(re.findall(r"if \(failed\) break;|return false;|&& landed;|&& !failed|if \(!failed\) failed|products_done, 0\)|q_full, 0\)|break;", text))
     assert waits >= 10 and ways_out >= waits - 3, (waits, ways_out)
+
+
+@pytest.mark.parametrize("name", ["attention_prefill_tc.cu", "differential_attention_tc.cu", "gemm_float_tc.cu"])
+def test_tensor_memory_is_taken_behind_the_wait_for_the_kernel_before(name):
+    text = SOURCES[name]
+    text = text[text.index("tcgen05.relinquish") - 2500 : text.index("tcgen05.relinquish")]
+    assert "pdl_wait();" in text[: text.index("tcgen05.alloc")], name
