@@ -332,6 +332,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
                 *failed = 1;
                 break;
             }
+            if (tile + pairs >= num_tiles) pdl_trigger();  // the main loop of this CTA's last tile is over
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * TILE_N;
             // four TMEM loads in flight before the one wait (32 gate and 32 up columns for the pair)
@@ -391,7 +392,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             if (lane == 0) mbar_arrive_cluster(empty_bar[acc]);
         }
     }
-    pdl_trigger();
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();

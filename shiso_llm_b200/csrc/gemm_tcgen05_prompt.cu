@@ -209,6 +209,7 @@ gemm_prompt_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
                 *failed = 1;
                 break;
             }
+            if (tile + (int)gridDim.x >= num_tiles) pdl_trigger();  // the main loop of this CTA's last tile is over
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + acc * TILE_N;
             // Four TMEM loads are in flight before the one wait: 64 columns a round (32 gate and
@@ -251,7 +252,6 @@ gemm_prompt_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_const
             if (lane == 0) mbar_arrive(&acc_empty[acc]);
         }
     }
-    pdl_trigger();
     __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();

@@ -58,3 +58,10 @@ def test_tensor_memory_is_taken_behind_the_wait_for_the_kernel_before(name):
     text = SOURCES[name]
     text = text[text.index("tcgen05.relinquish") - 2500 : text.index("tcgen05.relinquish")]
     assert "pdl_wait();" in text[: text.index("tcgen05.alloc")], name
+
+
+@pytest.mark.parametrize("name", ["gemm_tcgen05_prompt.cu", "gemm_tcgen05_pair.cu"])
+def test_products_let_their_successor_start_behind_their_main_loop(name):
+    """Not from lanes without a role, which come to the kernel's end at once."""
+    lines = [line.strip() for line in SOURCES[name].splitlines() if "pdl_trigger()" in line]
+    assert len(lines) == 1 and lines[0].startswith("if (tile + ") and ">= num_tiles) pdl_trigger();" in lines[0], lines
