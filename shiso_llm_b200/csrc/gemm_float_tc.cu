@@ -1,16 +1,20 @@
 // Y[T, N] = X[T, K] * W[N, K]^T (+ bias) in 32-bit floats on the tensor cores (tcgen05), from products of bfloat16
 // pieces.
 //
-// A float's 24 bits are three bfloat16 values h + m + l, each the eight leading bits of what the ones before
-// leave (cut off, not rounded: no piece overflows, and the sum is exact), and a product of two floats is the
-// sum of nine products of pieces, each exact in float.  The six largest are taken - hh, hm, mh, mm, hl, lh;
-// the others are below 2^-23 of the product together.  (bfloat16 ends at 2^-133, so an operand below 2^-110 keeps
-// that as an absolute error.)  The tensor core adds within a chunk of 64 columns,
-// the small products first and hh last, 4 additions deep; a chunk's sum is then added to a float register by an
-// ordinary addition, so that what the tensor core's own additions lose (they cut off) never grows with K.
+// A float is the sum of three bfloat16 values h + m + l, each what the ones before leave rounded to nearest (the sum is exact: the
+// rest behind two such roundings has seven bits; the splitting of floats for exact products is Dekker's, "A floating-point technique for
+// extending the available precision", 1971), and a product of two floats is the sum of nine products of pieces, each exact
+// in float.  The six largest are taken - hh, hm, mh, mm, hl, lh.  m is below 2^-8 and l below 2^-17 of its
+// float, of either sign, so the others are below 2^-24 of the product together, like the rounding of a multiply-add, and do not
+// add up over many products.  (bfloat16 ends at 2^-133, so an operand below 2^-110 keeps that as an absolute error.)  The tensor core
+// forms a chunk of 64 columns in 24 instructions, the small products first and hh in the last four; what its own additions lose (they
+// cut off, towards zero) is below 2^-21 of the products' magnitudes, and a chunk's sum is then added to a float register by an ordinary
+// addition, so that this never grows with K.
 //
-// Error against 64 bits, 2-norm over that of the result, normal operands: 1.3e-7 to 1.5e-7 for K 1,024 and 4,608, whatever N and the
-// rows; the multiply-adds of gemm_simple.cu 2.0e-7 (1,024 x 1,024), 3.1e-7 (1,024 x 4,608), 4.1e-7 (9,216 x 1,024), 5.8e-7 (65,536 x 1,024).
+// Error against 64 bits, 2-norm over that of the result, the multiply-adds of gemm_simple.cu first: operands of either sign 2.1e-7 and 1.0e-7 (300 x
+// 1,024 x 1,024), 3.2e-7 and 1.2e-7 (x 1,024 x 4,608), 4.1e-7 and 1.0e-7 (x 9,216 x 1,024), 5.7e-7 and 1.1e-7 (8 x 65,536 x 1,024). Where all products have
+// one sign what is cut off does not average out, 8.4e-8 of a result on average whatever the sizes: 2.5e-7 and 1.0e-7 (9,216 x
+// 1,024), but 0.8e-7 and 1.0e-7 (1,024 x 1,024), 0.9e-7 and 1.1e-7 (1,024 x 4,608). A result that one product dominates is right to 2^-22, by a multiply-add to 2^-24.
 //
 // A CTA has 128 rows of W (the MMA's M operand) x NT rows of X and walks one group of K, or all of them:
 //   warps 0-7    read the floats of W two chunks ahead (two 16-byte loads for eight columns of a row), split
@@ -22,19 +26,21 @@
 //                chunk's sums to its registers while the tensor core forms the next chunk's (two accumulators)
 // and warp 8 also issues the products, a chunk's before it adds the chunk's before (a seventeenth warp would leave 96
 // registers a thread instead of 128; issued by a splitting warp, which then splits late, 2,048 x 9,216 x 1,024 took 487 us).
-// Where a result is not finite (an infinity among the operands meets zeros among the other's pieces), it is formed
-// again as one chain of multiply-adds over its group, so infinities and NaN come out as from such a chain.
+// Where a result is not finite it is formed again as one chain of multiply-adds over its group, so infinities and NaN come out as
+// from such a chain.  (An infinity leaves a rest that is NaN, and so does a float that rounds up to one as a bfloat16, above 3.39e38: every
+// result that such an operand has a part in is formed again.)
 //
 // The order of a sum: chunks of 64 columns of a group in their order, groups in their order.  Groups are a
 // function of N and K alone, so a row's result depends neither on how many rows share the launch nor on
 // where it lies (gemm_simple.cu has the same property, with other bits).
 //
-// What bounds it: the instructions that split and add up - some 7,300 a chunk and CTA, beside 24 of the tensor
-// core, which is busy a fifth of the time (ncu, 300 x 9,216 x 1,024).
+// What bounds it: waits. Of the 17 cycles between two instructions of a warp nine go to loads and three to barriers, the schedulers issue in a
+// sixth of all cycles and the tensor core works in a quarter of the active ones (300 x 9,216 x 1,024; profiles/float_products.md);
+// that shape's 216 CTAs are one and a half for every SM.
 //
-// Measured, microseconds, gemm_simple.cu's first (rows x N x K): 1 x 9,216 x 1,024 40 and 16, 8 x 65,536 x 1,024 135 and 110, 1 x 1,024 x 4,608
-// 22 and 14, 24 x 9,216 x 1,024 70 and 19, 64 x 1,024 x 4,608 40 and 18, 300 x 9,216 x 1,024 182 and 109, 300 x 1,024 x 4,608 81 and 52, 300 x 1,024
-// x 1,024 26 and 23, 2,048 x 9,216 x 1,024 862 and 449.
+// Measured, microseconds, gemm_simple.cu's first (rows x N x K): 1 x 9,216 x 1,024 34 and 15, 8 x 65,536 x 1,024 133 and 105, 1 x 1,024 x 4,608
+// 17 and 13, 24 x 9,216 x 1,024 68 and 16, 64 x 1,024 x 4,608 38 and 17, 300 x 9,216 x 1,024 171 and 110, 300 x 1,024 x 4,608 81 and 51, 300 x 1,024
+// x 1,024 26 and 23, 2,048 x 9,216 x 1,024 861 and 457.  (With pieces that were cut off instead of rounded 300 x 9,216 x 1,024 took 109, 2,048 rows 449.)
 //
 // Every wait is bounded by a clock limit and reports through the status word.
 #include <type_traits>
@@ -63,26 +69,17 @@ struct FloatArgs {
 
 // Eight neighbouring floats as three words of eight bfloat16 each.
 __device__ __forceinline__ void split8(const float4& a, const float4& b, uint4 (&out)[3]) {
-    const float f[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-    uint32_t h[8], m[8], l[8];
+    float rest[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const uint32_t bits = __float_as_uint(f[i]);
-        const bool finite = fabsf(f[i]) < INFINITY;
-        h[i] = bits & 0xffff0000u;
-        if (!finite && (bits & 0x007fffffu)) h[i] |= 0x00400000u;  // (a NaN stays one)
-        const float rest = finite ? f[i] - __uint_as_float(h[i]) : 0.0f;
-        m[i] = __float_as_uint(rest) & 0xffff0000u;
-        l[i] = __float_as_uint(rest - __uint_as_float(m[i]));
-    }
-    uint32_t* o0 = reinterpret_cast<uint32_t*>(&out[0]);
-    uint32_t* o1 = reinterpret_cast<uint32_t*>(&out[1]);
-    uint32_t* o2 = reinterpret_cast<uint32_t*>(&out[2]);
+    for (int p = 0; p < 3; ++p) {
+        uint32_t* o = reinterpret_cast<uint32_t*>(&out[p]);
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        o0[i] = __byte_perm(h[2 * i], h[2 * i + 1], 0x7632);
-        o1[i] = __byte_perm(m[2 * i], m[2 * i + 1], 0x7632);
-        o2[i] = __byte_perm(l[2 * i], l[2 * i + 1], 0x7632);
+        for (int i = 0; i < 4; ++i) {
+            const __nv_bfloat162 pair = __floats2bfloat162_rn(rest[2 * i], rest[2 * i + 1]);
+            o[i] = *reinterpret_cast<const uint32_t*>(&pair);
+            rest[2 * i] -= __uint_as_float(o[i] << 16);
+            rest[2 * i + 1] -= __uint_as_float(o[i] & 0xffff0000u);
+        }
     }
 }
 

@@ -77,3 +77,58 @@ def test_float_products_that_are_not_finite(rows):
     keep = torch.ones(n, dtype=torch.bool)
     keep[[5, 9, 77]] = False
     assert torch.equal(got[3:][:, keep], clean[3:][:, keep])
+
+
+@pytest.mark.parametrize("k", [256, 1032, 4608])
+def test_float_products_whose_errors_do_not_average_out(k):
+    """Operands of one sign, and ones whose pieces leave as much as they can behind: most where they are rounded (1 + 2^-8 - 2^-17), and most
+    where they would be cut off (1 + 2^-7 - 2^-23).  What is left out of a product is below 2^-24 of it, and the 24 instructions of
+    a chunk cut off a unit of its sum at most in each of the last four, and of a 2^7th of it before: below 2^-21 of the result,
+    with the chunk sums' own rounding, K / 64 2^-25 of it on average."""
+    t = ops()
+    n, rows = 128, 40
+    w, x = rnd((n, k), torch.float32, 21).abs() + 0.1, rnd((rows, k), torch.float32, 22).abs() + 0.1
+    w[3], x[5] = 1 + 2.0 ** -7 - 2.0 ** -23, 1 + 2.0 ** -7 - 2.0 ** -23
+    w[4], x[6] = 1 + 2.0 ** -8 - 2.0 ** -17, -(1 + 2.0 ** -8 - 2.0 ** -17)
+    for part in (x, x[:9]):  # rows in pieces ahead of the product, and split by its own CTAs
+        got = t.linear(part.cuda().contiguous(), w.cuda(), torch.float32).cpu().double()
+        want = part.double() @ w.double().T
+        assert ((got - want) / want).abs().max() <= 2.0 ** -21 + k / 64 * 2.0 ** -25
+        if k > 1000:
+            chain = t.linear_simple(part.cuda().contiguous(), w.cuda(), torch.float32).cpu().double()
+            assert (got - want).norm() <= 1.05 * (chain - want).norm()
+
+
+def test_float_products_that_one_product_dominates():
+    """One column beside zeros, and beside columns 2^-40 as large: below 2^-24 of the product is left out and less than two units
+    cut off, 2^-22 together."""
+    t = ops()
+    n, k, rows = 192, 512, 24
+    w, x = rnd((n, k), torch.float32, 23), torch.zeros(rows, k)
+    x[:, 70] = rnd((rows,), torch.float32, 24)
+    x[rows // 2 :, 1:64] = rnd((rows - rows // 2, 63), torch.float32, 25) * 2.0 ** -40
+    got = t.linear(x.cuda(), w.cuda(), torch.float32).cpu().double()
+    want = x.double() @ w.double().T
+    large = want.abs() > 1e-3 * want.abs().max()  # (beside a tiny product the small columns are no longer small)
+    assert (((got - want) / want).abs()[large] <= 2.0 ** -22).all()
+
+
+@pytest.mark.parametrize("rows", [12, 24, 40])
+def test_floats_that_are_infinite_as_bfloat16(rows):
+    """Above 3.39e38 a float rounds up to an infinite bfloat16; beside infinities and NaN its results are formed again, and no other row is touched."""
+    t = ops()
+    n, k = 256, 1024
+    w, x = rnd((n, k), torch.float32, 13), rnd((rows, k), torch.float32, 14)
+    clean = t.linear(x.cuda(), w.cuda(), torch.float32).cpu()
+    x2 = x.clone()
+    x2[0] = 0.0
+    x2[0, 5], x2[1, 3], x2[2, 900] = 3.4e38, float("-inf"), float("nan")
+    w2 = w.clone()
+    w2[5, 70], w2[6] = float("inf"), w2[6].clamp(-0.9, 0.9)
+    got = t.linear(x2.cuda(), w2.cuda(), torch.float32).cpu()
+    chain = t.linear_simple(x2.cuda(), w2.cuda(), torch.float32).cpu()
+    assert torch.equal(torch.isnan(got), torch.isnan(chain)) and torch.equal(torch.isinf(got), torch.isinf(chain))
+    assert torch.equal(got[0, 6], chain[0, 6]) and torch.isfinite(got[0, 6])  # one product of a huge float and zeros: the chain's bits
+    keep = torch.ones(n, dtype=torch.bool)
+    keep[[5, 6]] = False
+    assert rows > 4 and torch.equal(got[3:][:, keep], clean[3:][:, keep])
