@@ -56,15 +56,16 @@ template <typename AT>
 __global__ void pool_kv_kernel(const AT* k_cache, const AT* v_cache, const int* table,
                                float* pooled_k, float* pooled_v, const int* pooled_table,
                                int table_width, const int* positions, const int* seq_of_token,
-                               int tokens, int kw, int vw, int page_size, int pool) {
-    // (few rows of a step end a block: a CTA looks through POOL_ROWS of them, columns are spread over blockIdx.y.  With a
+                               int tokens, int kw, int vw, int page_size, int pool, int rows) {
+    // (few rows of a step end a block: a CTA looks through `rows` of them, as many as a block has and at most POOL_ROWS, so that
+    // it finds one end of a sequence's, and columns are spread over blockIdx.y.  With a
     // row a CTA, 16,000 CTAs that mostly returned took 38 us for 2,000 rows.)
     __shared__ int ends[POOL_ROWS], found;
     if (threadIdx.x == 0) found = 0;
     __syncthreads();
     pdl_begin();
-    if (threadIdx.x < POOL_ROWS) {
-        const int t = blockIdx.x * POOL_ROWS + threadIdx.x;
+    if ((int)threadIdx.x < rows) {
+        const int t = blockIdx.x * rows + threadIdx.x;
         if (t < tokens && (positions[t] + 1) % pool == 0) ends[atomicAdd(&found, 1)] = t;
     }
     __syncthreads();
@@ -84,7 +85,7 @@ __global__ void pool_kv_kernel(const AT* k_cache, const AT* v_cache, const int* 
                 float v[16];
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
-                    const int p = min(p0 + j, pos), page = pages[p / page_size];
+                    const int p = p0 + j, page = p <= pos ? pages[p / page_size] : -1;
                     v[j] = page < 0 ? 0.0f : to_f32(cache[((size_t)page * page_size + p % page_size) * width + col]);
                 }
 #pragma unroll
@@ -102,14 +103,15 @@ SHISO_API int shiso_pool_kv(const void* k_cache, const void* v_cache, int cache_
                             cudaStream_t stream) {
     if (tokens <= 0) return SHISO_OK;
     if (pool < 1) return SHISO_ERR_SHAPE;
-    const dim3 grid(ceil_div_u(tokens, POOL_ROWS), ceil_div_u((long long)kv_heads * (dim + vdim), 128) < 16 ? ceil_div_u((long long)kv_heads * (dim + vdim), 128) : 16);
+    const int rows = pool < POOL_ROWS ? pool : POOL_ROWS;
+    const dim3 grid(ceil_div_u(tokens, rows), ceil_div_u((long long)kv_heads * (dim + vdim), 128) < 16 ? ceil_div_u((long long)kv_heads * (dim + vdim), 128) : 16);
     if (cache_dtype == SHISO_F32)
         launch_kernel(pool_kv_kernel<float>, grid, 128, 0, stream, (const float*)k_cache, (const float*)v_cache, table, pooled_k,
-                      pooled_v, pooled_table, table_width, positions, seq_of_token, tokens, kv_heads * dim, kv_heads * vdim, page_size, pool);
+                      pooled_v, pooled_table, table_width, positions, seq_of_token, tokens, kv_heads * dim, kv_heads * vdim, page_size, pool, rows);
     else if (cache_dtype == SHISO_BF16)
         launch_kernel(pool_kv_kernel<__nv_bfloat16>, grid, 128, 0, stream, (const __nv_bfloat16*)k_cache,
                       (const __nv_bfloat16*)v_cache, table, pooled_k, pooled_v, pooled_table, table_width, positions, seq_of_token,
-                      tokens, kv_heads * dim, kv_heads * vdim, page_size, pool);
+                      tokens, kv_heads * dim, kv_heads * vdim, page_size, pool, rows);
     else
         return SHISO_ERR_DTYPE;
     return launch_status();
