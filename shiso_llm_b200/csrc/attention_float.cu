@@ -2,7 +2,7 @@
 //
 // The general kernel (attention.cu) has a warp per (row, head) whose lanes each read a key row of their
 // own, 256 bytes apart: every load is 32 sectors, every row reads all its keys again, and 300 rows of 16
-// heads took 477 us for what is 0.2 GFLOP.  Here a CTA takes 32 query rows of one sequence and one head;
+// heads of 64 took 286 us for what is 0.2 GFLOP.  Here a CTA takes 32 query rows of one sequence and one head;
 // tiles of 32 keys and their values come to shared memory once (16-byte cp.async through the block table, two
 // stages), a thread has 2 rows x 4 keys of the scores and then 4 rows x HEAD / 16 columns of the output.
 //

@@ -118,7 +118,7 @@ __global__ void short_conv_out_vec_kernel(const __nv_bfloat16* proj, const float
 // it.  Per channel the sum is the same fused multiply-adds in the same order as above.
 
 // A run's refills are what it waits for where many sequences begin in it, and a step's longest run ends last:
-// steps of several sequences take runs of four rows (2,048 channels, microseconds with runs of 16 and of four:
+// steps of eight sequences and more take runs of four rows (2,048 channels, microseconds with runs of 16 and of four:
 // 32 single rows beside 1,024 14.5 and 8.7, 64 beside 512 14.5 and 7.7, eight portions of 100 8.1 and 6.7).
 constexpr int LONG_RUN = 16, SHORT_RUN = 4, SHORT_RUN_SEQS = 8;
 
@@ -372,9 +372,9 @@ SHISO_API int shiso_short_conv(const void* proj, int act_dtype, const float* w, 
                          (((uintptr_t)proj | (uintptr_t)y | (uintptr_t)state) & 15) == 0;
         const bool runs = vec && tokens >= 512 && taps >= 2 && taps <= 4;
         if (runs) {
-            const bool few = seqs >= SHORT_RUN_SEQS;
+            const bool many = seqs >= SHORT_RUN_SEQS;  // sequences
             auto launch_run = [&](auto long_kernel, auto short_kernel) {
-                launch_kernel(few ? short_kernel : long_kernel, dim3(ceil_div_u(tokens, few ? SHORT_RUN : LONG_RUN), ceil_div_u(hidden / 8, threads)), threads, 0, stream, (const __nv_bfloat16*)proj, w, bias,
+                launch_kernel(many ? short_kernel : long_kernel, dim3(ceil_div_u(tokens, many ? SHORT_RUN : LONG_RUN), ceil_div_u(hidden / 8, threads)), threads, 0, stream, (const __nv_bfloat16*)proj, w, bias,
                               (const float*)state, slot_stride, seq_of_token, q_start, slots, (__nv_bfloat16*)y, hidden, tokens);
             };
             if (taps == 2) launch_run(short_conv_run_kernel<2, LONG_RUN>, short_conv_run_kernel<2, SHORT_RUN>);

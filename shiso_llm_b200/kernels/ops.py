@@ -1021,11 +1021,7 @@ def paged_attention(q, heads, kv_heads, head_dim, k_cache, v_cache, block_table,
         _done(status, "prefill_attention (tcgen05)", shape=(tokens, heads, head_dim))
         return out
     elif q.dtype == torch.bfloat16 and head_dim % 16 == 0 and head_dim <= PREFILL_MAX_HEAD_DIM:
-        starts = getattr(step, "h_q_start", None)
-        if starts:
-            tiles = sum(-(-(b - a) // 64) for a, b in zip(starts[:-1], starts[1:]))
-        else:
-            tiles = tokens // 64 + step.num_seqs
+        tiles = _portion_tiles(step, tokens, 64)
         status = lib.shiso_prefill_attention(
             _ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(block_table), block_table.shape[1], _ptr(step.q_start),
             _ptr(step.start_pos), _ptr(out), step.num_seqs, tiles, heads, kv_heads, head_dim, page_size,
@@ -1559,11 +1555,7 @@ def masked_attention(q, heads, k_cache, v_cache, block_table, page_size, scale, 
         not general and act == torch.bfloat16 and not getattr(step, "all_decode", False)
         and lib.shiso_masked_attention_tiles_supported(dim, vdim)
     ):
-        starts = getattr(step, "h_q_start", None)
-        if starts:
-            tiles = sum(-(-(b - a) // 64) for a, b in zip(starts[:-1], starts[1:]))
-        else:
-            tiles = tokens // 64 + step.num_seqs
+        tiles = _portion_tiles(step, tokens, 64)
         status = lib.shiso_masked_attention_tiles(
             q.data_ptr(), q_ld, _ptr(k_cache), _ptr(v_cache), _ptr(block_table), block_table.shape[1], _ptr(step.q_start),
             _ptr(step.start_pos), _ptr(out), heads * vdim, gate.data_ptr() if gate is not None else 0, gate_ld, _ptr(key_bias),
@@ -1646,11 +1638,7 @@ def differential_attention(q, pairs, groups, k_cache, v_cache, block_table, page
             k_cache.shape[0], float(scale), window, splits, float(second), float(factor), float(eps), _stream())
         _done(status, "differential_attention (decode)", shape=(tokens, pairs, dim))
         return out
-    starts = getattr(step, "h_q_start", None)
-    if starts:
-        tiles = sum(-(-(b - a) // 128) for a, b in zip(starts[:-1], starts[1:]))
-    else:
-        tiles = tokens // 128 + step.num_seqs
+    tiles = _portion_tiles(step, tokens, 128)
     status = lib.shiso_differential_prefill(
         q.data_ptr(), q_ld, _ptr(k_cache), _ptr(v_cache), _ptr(block_table), block_table.shape[1], _ptr(step.q_start), _ptr(step.start_pos),
         gate.data_ptr(), gate_ld, out.data_ptr(), out_ld, tokens, step.num_seqs, tiles, pairs, groups, dim, vdim, page_size, k_cache.shape[0],
@@ -2140,8 +2128,6 @@ def head_linear(x, w, out, gate=None):
 
 LATENT_DECODE_SHARE_KEYS = 256  # a decode step's keys are shared out over CTAs in ranges of about this many (a run of 32 per warp) ...
 LATENT_MAX_SHARES = 16  # ... up to this many CTAs a (row, head group)
-
-
 LATENT_MMA_MIN_PORTION = 8  # steps whose longest portion has at least this many rows take the tensor-core kernel (bfloat16)
 
 
@@ -2163,11 +2149,7 @@ def latent_attention(q_lat, rank, k_cache, block_table, page_size, scale, step, 
         not general and q_lat.dtype == torch.bfloat16 and not getattr(step, "all_decode", False)
         and getattr(step, "max_q_len", tokens) >= LATENT_MMA_MIN_PORTION and lib.shiso_latent_prefill_supported(int(rank), width)
     ):
-        starts = getattr(step, "h_q_start", None)
-        if starts:
-            tiles = sum(-(-(b - a) // 16) for a, b in zip(starts[:-1], starts[1:]))
-        else:
-            tiles = tokens // 16 + step.num_seqs
+        tiles = _portion_tiles(step, tokens, 16)
         status = lib.shiso_latent_prefill(
             _ptr(q_lat), _ptr(k_cache), _ptr(block_table), block_table.shape[1], _ptr(step.q_start), _ptr(step.start_pos), _ptr(out),
             step.num_seqs, tiles, heads, int(rank), width, page_size, float(scale), _stream(),
