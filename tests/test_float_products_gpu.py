@@ -132,3 +132,32 @@ def test_floats_that_are_infinite_as_bfloat16(rows):
     keep = torch.ones(n, dtype=torch.bool)
     keep[[5, 6]] = False
     assert rows > 4 and torch.equal(got[3:][:, keep], clean[3:][:, keep])
+
+
+@pytest.mark.parametrize("n,k,rows", [(128, 16384, 20), (300, 4608, 130), (129, 1032, 17), (4608, 520, 65)])
+def test_groups_with_ctas_of_their_own_have_the_bits_of_one_cta(n, k, rows):
+    t = ops()
+    lib, sums = t.library(), {}
+    w, x, bias = rnd((n, k), torch.float32, 1).cuda(), rnd((rows, k), torch.float32, 3).cuda(), rnd((n,), torch.float32, 2).cuda()
+    group = -(-lib.shiso_gemm_float_group_columns(n, k) // 64) * 64
+    pieces = torch.empty(3, rows, k, dtype=torch.bfloat16, device="cuda")
+    for split in (False, True):
+        sums[split] = torch.empty(rows, n, device="cuda")
+        partial = torch.empty(-(-k // group), rows, n, device="cuda")
+        assert lib.shiso_gemm_float_tc(x.data_ptr(), w.data_ptr(), bias.data_ptr(), sums[split].data_ptr(), partial.data_ptr() if split else 0,
+                                       pieces.data_ptr(), rows, n, k, group, torch.cuda.current_stream().cuda_stream) == 0
+    assert torch.equal(sums[False], sums[True]) and torch.equal(sums[True], t.linear(x, w, torch.float32, bias))
+
+
+@pytest.mark.parametrize("n,k,rows", [(4608, 4612, 630), (512, 4100, 4600), (128, 16388, 700)])
+def test_products_that_stay_with_the_multiply_adds(n, k, rows):
+    """Columns of 4 modulo 8 are no whole bfloat16 words: groups that one CTA walks, groups whose sums would take more room than is set
+    aside, and as many groups as there are, with the bits of the other form."""
+    t = ops()
+    w, x = rnd((n, k), torch.float32, 1).cuda(), rnd((rows, k), torch.float32, 3).cuda()
+    assert not t.library().shiso_gemm_float_tc_supported(x.data_ptr(), w.data_ptr(), x.data_ptr(), rows, n, k)
+    groups = lambda r: t.library().shiso_gemm_float_groups(x.data_ptr(), w.data_ptr(), x.data_ptr(), r, n, k, t._sm_count())
+    full = t.linear(x, w, torch.float32)
+    assert groups(64) >= 2 and (groups(rows) > 0) == (k == 16388)
+    for a, part in ((0, 64), (5, 1), (100, 20), (300, 250)):
+        assert torch.equal(t.linear(x[a : a + part].contiguous(), w, torch.float32), full[a : a + part]), (a, part)
