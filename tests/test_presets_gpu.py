@@ -1,0 +1,70 @@
+"""Presets at their real widths (their first layers): prompts read in captured steps that follow one another without a wait, each
+model behind the others in one process, as a server or a benchmark has them.  Every pass has the first one's bits, no bounded wait runs out, and
+no pass takes longer than the host's limit."""
+
+import json
+import time
+
+import numpy as np
+import pytest
+import torch
+
+from shiso_llm_b200 import Engine, EngineOptions, StepEntry
+from shiso_llm_b200.cli import preset_path
+from shiso_llm_b200.config import plan_from_document
+from shiso_llm_b200.parts import BuildEnv, Model
+from shiso_llm_b200.weights import random_device_tensors
+
+pytestmark = pytest.mark.gpu
+
+LIMIT_S = 30.0  # a pass takes milliseconds
+
+
+def settle(what):
+    event, began = torch.cuda.Event(), time.monotonic()
+    event.record()
+    while not event.query():
+        assert time.monotonic() - began < LIMIT_S, f"{what}: the device did not come to the end of it"
+        time.sleep(0.001)
+
+
+@pytest.mark.parametrize("preset,dtype,layers,tokens", [
+    ("lfm2-1.2b", "bfloat16", 0, 700), ("lfm2-350m", "float32", 0, 300), ("volalorn-1b", "bfloat16", 6, 1501), ("filulix-1b", "bfloat16", 6, 1300),
+    ("zetavik-1b", "bfloat16", 6, 600), ("povilorn-350m", "bfloat16", 9, 1100), ("nodepel-350m", "bfloat16", 8, 500), ("raketar-350m", "bfloat16", 8, 500),
+    ("lfm2-350m", "float32", 0, 24), ("volalorn-350m", "bfloat16", 16, 700),
+])
+def test_prompts_of_presets_one_behind_the_other(preset, dtype, layers, tokens):
+    from shiso_llm_b200.kernels import ops
+
+    with open(preset_path(preset)) as f:
+        document = json.load(f)
+    if layers:
+        document["layers"] = document["layers"][:layers]
+    _, _, plan = plan_from_document(document)
+    device = torch.device("cuda:0")
+    model = Model(plan, BuildEnv(dtype=getattr(torch, dtype), device=device, ops=ops))
+    weights = random_device_tensors(model.tensor_specs(), 1, getattr(torch, dtype), device)
+    engine = Engine.from_plan(plan, weights, EngineOptions(dtype=dtype, ctx=2048, page_size=16, kv_cache_tokens=6144, max_num_seqs=8,
+                                                           max_num_batched_tokens=tokens + 64))
+    rng = np.random.RandomState(3)
+    prompt = rng.randint(0, plan.vocab_size, tokens).tolist()
+    running = [rng.randint(0, plan.vocab_size, 120).tolist() for _ in range(6)]
+
+    def read(turn):
+        logits = engine.step([StepEntry(("p", turn), prompt, [tokens - 1])])
+        engine.finish(("p", turn))
+        return logits
+
+    first = [read(i).clone() for i in range(3)][-1]  # kernel by kernel, captured, replayed
+    for turn in range(3, 63):
+        last = read(turn)
+    settle(f"{preset}: 60 prompts")
+    assert torch.isfinite(first).all() and torch.equal(first, last)
+    for i, t in enumerate(running):
+        engine.step([StepEntry(("r", i), t[:60], [])])
+    for at in range(60, 90):  # a portion beside requests that decode, in the same shape again and again
+        logits = engine.step([StepEntry(("r", i), [t[at]], [0]) for i, t in enumerate(running)] + [StepEntry(("p", at), prompt[: tokens // 2], [tokens // 2 - 1])])
+        engine.finish(("p", at))
+    settle(f"{preset}: 30 portions beside decoding requests")
+    assert torch.isfinite(logits).all()
+    ops.check_kernel_status()
