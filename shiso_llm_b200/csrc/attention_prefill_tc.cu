@@ -166,9 +166,6 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         mbar_init(products_done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
-    pdl_wait();  // queries, keys and values were written by the kernels before this one
-    if (threadIdx.x == 0) {
         shared_ints[0] = 0;
         // which (sequence, tile) is this CTA?  The last tiles of a portion have the most keys:
         // they take the first CTAs - of every head, the head being the grid's fast index - so
@@ -191,14 +188,6 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     __syncthreads();
     const int seq = shared_ints[1];
     if (seq < 0) return;  // uniform: before any TMEM allocation
-    if (warp == 5) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem_base = *tmem_slot;
 
     const int row0 = shared_ints[2];
     const int first_token = a.q_start[seq] + row0;
@@ -214,6 +203,19 @@ flash_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     const int num_tiles = kept_tiles + tile_last - tile_first + 1;
     auto tile_at = [&](int it) { return it < kept_tiles ? it : tile_first - kept_tiles + it; };
     bool failed = false;
+
+    pdl_wait();  // queries, keys and values were written by the kernels before this one
+    uint32_t tmem_base = 0;
+    if (warp != 4) {  // (the producer needs none, and its first copies travel meanwhile)
+        if (warp == 5) {
+            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
+            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        asm volatile("bar.sync 1, %0;" ::"n"(THREADS - 32) : "memory");
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        tmem_base = *tmem_slot;
+    }
 
     if (warp == 4) {
         // ---- producer: lane p brings page p of every tile (its key box and its value box), and

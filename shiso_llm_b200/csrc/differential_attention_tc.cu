@@ -148,9 +148,6 @@ differential_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
         mbar_init(products_done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    }
-    pdl_wait();  // queries, keys and values were written by the kernels before this one
-    if (threadIdx.x == 0) {
         shared_ints[0] = 0;
         // the last tiles of a portion have the most keys: they take the first CTAs of every head
         int left = gridDim.y - 1 - blockIdx.y, found = -1, row0 = 0;
@@ -169,6 +166,7 @@ differential_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     __syncthreads();
     const int seq = shared_ints[1];
     if (seq < 0) return;  // uniform: before any TMEM allocation
+    pdl_wait();  // queries, keys and values were written by the kernels before this one
     if (warp == 9) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS) : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
