@@ -2,8 +2,8 @@
 // pieces.
 //
 // A float is the sum of three bfloat16 values h + m + l, each what the ones before leave rounded to nearest (the sum is exact: the
-// rest behind two such roundings has seven bits; the splitting of floats for exact products is Dekker's, "A floating-point technique for
-// extending the available precision", 1971), and a product of two floats is the sum of nine products of pieces, each exact
+// rest behind two such roundings has seven bits; the method is Henry, Tang and Heinecke's, "Leveraging the bfloat16 artificial
+// intelligence datatype for higher-precision computations", 2019), and a product of two floats is the sum of nine products of pieces, each exact
 // in float.  The six largest are taken - hh, hm, mh, mm, hl, lh.  m is below 2^-8 and l below 2^-17 of its
 // float, of either sign, so the others are below 2^-24 of the product together, like the rounding of a multiply-add, and do not
 // add up over many products.  (bfloat16 ends at 2^-133, so an operand below 2^-110 keeps that as an absolute error.)  The tensor core
