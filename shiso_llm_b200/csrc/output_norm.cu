@@ -112,7 +112,8 @@ __global__ void norm_into_vec_kernel(float* residual, const __nv_bfloat16* y, co
 }
 
 // A row stays in registers between its statistics and its result (Q pieces of eight a thread), and the three
-// sums meet in one pass through shared memory, each in block_sum's order.  The row's traffic bounds it.
+// sums meet in one pass through shared memory, each in block_sum's order; rows of more than 32,768 entries (Q = 0) are read twice.  The
+// row's traffic bounds it.
 // (The row read twice and three sums one after the other, microseconds, and this: 1,501 rows of 8,448 14.2 and 12.5, 300 6.0 and
 // 5.2, 8 3.2 and 2.6; 512 of 4,608 5.0 and 4.3.)
 template <int Q>
@@ -122,17 +123,10 @@ __global__ void __launch_bounds__(512) polynorm_vec_kernel(const __nv_bfloat16* 
     pdl_begin();
     const int pieces = width >> 3, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const uint4* src = reinterpret_cast<const uint4*>(z + (size_t)blockIdx.x * z_ld);
-    uint4 raw[Q];
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-        const int i = threadIdx.x + q * blockDim.x;
-        raw[q] = i < pieces ? src[i] : make_uint4(0u, 0u, 0u, 0u);
-    }
     float sums[3] = {0.0f, 0.0f, 0.0f};
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
+    auto add = [&](const uint4& piece) {
         float v[8];
-        unpack8(raw[q], v);
+        unpack8(piece, v);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             const float v2 = v[e] * v[e];
@@ -140,6 +134,18 @@ __global__ void __launch_bounds__(512) polynorm_vec_kernel(const __nv_bfloat16* 
             sums[1] += v2 * v2;
             sums[2] += v2 * v2 * v2;
         }
+    };
+    uint4 raw[Q > 0 ? Q : 1];
+    if constexpr (Q > 0) {
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+            const int i = threadIdx.x + q * blockDim.x;
+            raw[q] = i < pieces ? src[i] : make_uint4(0u, 0u, 0u, 0u);
+        }
+#pragma unroll
+        for (int q = 0; q < Q; ++q) add(raw[q]);
+    } else {
+        for (int i = threadIdx.x; i < pieces; i += blockDim.x) add(src[i]);
     }
 #pragma unroll
     for (int i = 0; i < 3; ++i) {
@@ -154,14 +160,18 @@ __global__ void __launch_bounds__(512) polynorm_vec_kernel(const __nv_bfloat16* 
     const float c = coefficients[2] * rsqrtf(sums[2] / (float)width + eps);
     const float e0 = coefficients[3];
     uint4* dst = reinterpret_cast<uint4*>(out + (size_t)blockIdx.x * width);
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-        const int i = threadIdx.x + q * blockDim.x;
+    auto put = [&](int i, const uint4& piece) {
         float v[8];
-        unpack8(raw[q], v);
+        unpack8(piece, v);
 #pragma unroll
         for (int e = 0; e < 8; ++e) v[e] = a * v[e] + b * (v[e] * v[e]) + c * (v[e] * v[e] * v[e]) + e0;
         if (i < pieces) dst[i] = pack8(v);
+    };
+    if constexpr (Q > 0) {
+#pragma unroll
+        for (int q = 0; q < Q; ++q) put(threadIdx.x + q * blockDim.x, raw[q]);
+    } else {
+        for (int i = threadIdx.x; i < pieces; i += blockDim.x) put(i, src[i]);
     }
 }
 
@@ -311,7 +321,7 @@ SHISO_API int shiso_polynorm(const void* z, long long z_ld, int act_dtype, const
     if (width <= 0) return SHISO_ERR_SHAPE;
     if (act_dtype == SHISO_F32)
         launch_kernel(polynorm_kernel<float>, tokens, block_for(width), 0, stream, (const float*)z, z_ld, coefficients, (float*)out, width, eps);
-    else if (act_dtype == SHISO_BF16 && width % 8 == 0 && width <= 32768 && z_ld % 8 == 0 && aligned16(z, out, nullptr, nullptr)) {
+    else if (act_dtype == SHISO_BF16 && width % 8 == 0 && z_ld % 8 == 0 && aligned16(z, out, nullptr, nullptr)) {
         const int threads = width > 16384 ? 512 : (width > 4096 ? 256 : 128), q = ceil_div_u(width / 8, threads);
         auto go = [&](auto kernel) {
             launch_kernel(kernel, tokens, threads, 0, stream, (const __nv_bfloat16*)z, z_ld, coefficients, (__nv_bfloat16*)out, width, eps);
@@ -320,7 +330,8 @@ SHISO_API int shiso_polynorm(const void* z, long long z_ld, int act_dtype, const
         else if (q <= 2) go(polynorm_vec_kernel<2>);
         else if (q <= 4) go(polynorm_vec_kernel<4>);
         else if (q <= 5) go(polynorm_vec_kernel<5>);
-        else go(polynorm_vec_kernel<8>);
+        else if (q <= 8) go(polynorm_vec_kernel<8>);
+        else go(polynorm_vec_kernel<0>);
     }
     else if (act_dtype == SHISO_BF16)
         launch_kernel(polynorm_kernel<__nv_bfloat16>, tokens, block_for(width), 0, stream, (const __nv_bfloat16*)z, z_ld, coefficients,

@@ -9,10 +9,10 @@ from test_kernels_gpu import close, make_step, ops, rnd
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("width", [1032, 2048, 4096, 4104, 4608, 8448, 10240, 16384, 16392, 32768, 32776])
+@pytest.mark.parametrize("width", [1032, 2048, 4096, 4104, 4608, 8448, 10240, 16384, 16392, 32768, 32776, 50008])
 def test_polynorm_widths(width):
-    """Pieces of eight a thread: 1, 2, 4, 5 and 8, with 128, 256 and 512 threads; wider rows and rows off 16-byte boundaries take
-    the general kernel, whose sums run in another order."""
+    """Pieces of eight a thread: 1, 2, 4, 5 and 8, with 128, 256 and 512 threads, and wider rows, read twice; rows off 16-byte
+    boundaries take the general kernel, whose sums run in another order."""
     z, c = rnd((5, width + 8), torch.bfloat16, width), torch.tensor([0.7, -0.4, 0.2, 0.1])
     for first in (0, 1):  # (a column range that starts off a 16-byte boundary)
         view = z[:, first : first + width]
