@@ -93,7 +93,10 @@ __global__ void __launch_bounds__(LA_WARPS * 32) latent_attention_kernel(
         const AT* row = cache + at;
         float s[LA_HEADS] = {};
         if (VEC) {
-            constexpr int N = LaVec<AT>::N, AHEAD = RV > 8 ? 2 : 8;  // words of the row asked for together: a decode step's few warps wait for nothing else
+            constexpr int N = LaVec<AT>::N;
+            // words of the row asked for together: a decode step's few warps wait for nothing else.  (A latent of more than 256 leaves no
+            // registers for it: eight rows of four heads of 512 / 576 at 1,500 83 us with one word, 87 with two.)
+            constexpr int AHEAD = RV > 8 ? 1 : 8;
             for (int d0 = 0; d0 < width; d0 += N * AHEAD) {
                 uint4 raw[AHEAD];
 #pragma unroll
