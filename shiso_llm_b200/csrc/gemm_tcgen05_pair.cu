@@ -207,7 +207,8 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     uint64_t* empty = full + STAGES;
     uint64_t* acc_full = empty + STAGES;   // [2]
     uint64_t* acc_empty = acc_full + 2;    // [2]
-    uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
+    uint64_t* peer_ready = acc_empty + 2;  // (used in the leader) the peer has its tensor memory
+    uint32_t* tmem_slot = (uint32_t*)(peer_ready + 1);
     int* failed = (int*)(tmem_slot + 1);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -227,52 +228,72 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
             mbar_init(&acc_full[i], 1);   // one commit
             mbar_init(&acc_empty[i], 8);  // four epilogue warps in each CTA (used in the leader)
         }
+        mbar_init(peer_ready, 1);
         *failed = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     }
-    if (warp == 1) {
-        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     cluster_sync_all();  // the peer's barriers exist before anything is signalled on them
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t tmem_base = *tmem_slot;
+
+    // Tensor memory is taken behind the wait for the kernel before, when nothing else on the device holds any or gives some back.  (Ahead of
+    // it, under the tail of the kernels before, one CTA of a pair could wait for its allocation for ever, its peer's having returned and
+    // nobody holding any: after ten to some hundred replays of a step of 1,984 rows.)  The permit to allocate is the pair's and is kept to the end.
+    uint32_t tmem_base = 0;
+    if (warp != 0) {
+        pdl_wait();
+        if (warp == 1) {
+            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
+        }
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+        asm volatile("bar.sync 1, %0;" ::"n"(THREADS - 32) : "memory");
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        tmem_base = *tmem_slot;
+    }
 
     if (warp == 0) {
         if (lane == 0) {
-            // ---- producer of this CTA's halves
+            // ---- producer of this CTA's halves.  Weights depend on no predecessor, the activations do: the weights of every
+            // stage of the ring are asked for ahead of the wait.
+            auto load_weights = [&](int s, int kb, int w_row) {
+                if (leader) mbar_expect_tx(&full[s], 2 * STAGE_BYTES);
+                tma_load_2d_pair(smem + s * STAGE_BYTES + A_BYTES, &map_w, kb * BK, w_row, peer_address(smem_u32(&full[s]), 0));
+            };
+            auto load_tokens = [&](int s, int kb, int m0) {
+                tma_load_2d_pair(smem + s * STAGE_BYTES, &map_x, kb * BK, m0, peer_address(smem_u32(&full[s]), 0));
+            };
             int it = 0;
             bool ok = true;
             for (int tile = pair; tile < num_tiles && ok; tile += pairs) {
                 const int m0 = (tile % p.m_tiles) * (2 * HALF_M) + (int)rank * HALF_M;
                 const int n_tile0 = (tile / p.m_tiles) * out_per_tile;
                 const int w_row = GLU ? (leader ? n_tile0 : p.inter + n_tile0) : n_tile0 + (int)rank * HALF_N;
-                for (int kb = 0; kb < k_blocks; ++kb, ++it) {
+                if (it == 0) {
+                    const int ahead = min(k_blocks, STAGES);
+                    for (int kb = 0; kb < ahead; ++kb) load_weights(kb, kb, w_row);
+                    pdl_wait();
+                    for (; it < ahead; ++it) load_tokens(it, it, m0);
+                }
+                for (int kb = tile == pair ? it : 0; kb < k_blocks; ++kb, ++it) {
                     const int s = it % STAGES;
                     if (it >= STAGES && !mbar_wait(&empty[s], ((it / STAGES) - 1) & 1)) {
                         *failed = 1;
                         ok = false;
                         break;
                     }
-                    uint8_t* a = smem + s * STAGE_BYTES;
-                    const uint32_t bar = peer_address(smem_u32(&full[s]), 0);
-                    if (leader) mbar_expect_tx(&full[s], 2 * STAGE_BYTES);
-                    const int k = kb * BK;
-                    tma_load_2d_pair(a + A_BYTES, &map_w, k, w_row, bar);
-                    if (it == 0) pdl_wait();  // weights depend on no predecessor; the activations do
-                    tma_load_2d_pair(a, &map_x, k, m0, bar);
+                    load_weights(s, kb, w_row);
+                    load_tokens(s, kb, m0);
                 }
             }
         }
     } else if (warp == 1) {
+        if (lane == 0 && !leader) mbar_arrive_cluster(peer_address(smem_u32(peer_ready), 0));
         if (lane == 0 && leader) {
             // ---- MMA issuer of the pair
             const uint32_t idesc = umma_idesc(2 * HALF_M, TILE_N);
             int it = 0, local = 0;
-            bool ok = true;
+            bool ok = mbar_wait_cluster(peer_ready, 0);
+            if (!ok) *failed = 1;
             for (int tile = pair; tile < num_tiles && ok; tile += pairs, ++local) {
                 const int acc = local & 1;
                 if (local >= 2 && !mbar_wait_cluster(&acc_empty[acc], ((local >> 1) - 1) & 1)) {
@@ -302,7 +323,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
         }
     } else {
         // ---- epilogue warps 2..5: TMEM lanes (warp % 4) * 32 .., one token per thread
-        pdl_wait();
         const int quarter = warp & 3;
         const uint32_t empty_bar[2] = {peer_address(smem_u32(&acc_empty[0]), 0), peer_address(smem_u32(&acc_empty[1]), 0)};
         int local = 0;
@@ -398,8 +418,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constan
     if (*failed != 0 && threadIdx.x == 0 && p.status) atomicExch(p.status, 1);
     cluster_sync_all();  // nobody signals into, or frees, a CTA that a peer still uses
     if (warp == 1) {
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
         asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(512) : "memory");
     }
+    cluster_sync_all();  // both free the pair's tensor memory before either ends
 }
 
 template <bool GLU>

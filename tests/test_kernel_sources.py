@@ -65,3 +65,15 @@ def test_products_let_their_successor_start_behind_their_main_loop(name):
     """Not from lanes without a role, which come to the kernel's end at once."""
     lines = [line.strip() for line in SOURCES[name].splitlines() if "pdl_trigger()" in line]
     assert len(lines) == 1 and lines[0].startswith("if (tile + ") and ">= num_tiles) pdl_trigger();" in lines[0], lines
+
+
+def test_a_pair_takes_and_gives_back_its_tensor_memory_when_nothing_else_does():
+    """Ahead of the wait for the kernel before, one CTA's allocation could stand for ever.  Both CTAs free theirs before either ends."""
+    assert [name for name, t in SOURCES.items() if "tcgen05.alloc.cta_group::2" in t] == ["gemm_tcgen05_pair.cu"]
+    text = SOURCES["gemm_tcgen05_pair.cu"]
+    text = text[text.index("gemm_pair_kernel("):]
+    order = [text.index(x) for x in ("cluster_sync_all();", "pdl_wait();", "tcgen05.alloc.cta_group::2", "// ---- producer", "// ---- epilogue",
+                                     "nobody signals into", "tcgen05.relinquish_alloc_permit.cta_group::2", "tcgen05.dealloc.cta_group::2")]
+    assert order == sorted(order)
+    behind = text[order[-1]:]
+    assert "cluster_sync_all();" in behind[: behind.index("\n}\n")]
