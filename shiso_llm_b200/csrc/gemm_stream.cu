@@ -228,15 +228,19 @@ gemm_stream_kernel(StreamArgs a) {
             const __nv_bfloat16* src = a.w + (size_t)(row >= 0 ? row : 0) * a.K;
             for (int c = 0; c < chunks; ++c, ++unit) {
                 const int s = unit % STAGES;
-                if (unit >= STAGES && !mbar_wait(&empty[s], ((unit / STAGES) - 1) & 1)) timed_out = true;
+                if (unit >= STAGES && !timed_out && !mbar_wait(&empty[s], ((unit / STAGES) - 1) & 1)) timed_out = true;  // (no other is begun, nothing more is copied)
                 const int cols = min(KC, a.K - c * KC);
-                if (lane == 0) mbar_expect_tx(&full[s], (uint32_t)(present * cols * 2));
+                if (lane == 0 && !timed_out) mbar_expect_tx(&full[s], (uint32_t)(present * cols * 2));
                 __syncwarp();
-                if (row >= 0)
+                if (row >= 0 && !timed_out)
                     bulk_load(smem_u32(ring + s * STAGE_BYTES) + lane * ROW_BYTES, src + (size_t)c * KC, (uint32_t)(cols * 2), &full[s]);
             }
         }
-        if (timed_out && lane == 0 && a.status) atomicExch(a.status, 1);
+        if (timed_out) {  // no consumer may wait for them any more: the last copies land before the CTA ends
+            for (int u = max(0, unit - STAGES); u < unit; ++u)
+                if (!mbar_wait(&full[u % STAGES], (u / STAGES) & 1)) break;
+            if (lane == 0 && a.status) atomicExch(a.status, 1);
+        }
         pdl_trigger();
         return;
     }
@@ -343,7 +347,7 @@ gemm_stream_kernel(StreamArgs a) {
         // one stage: wait for it, multiply this warp's columns, give it back
         auto work = [&](int c, uint4 (&xv)[KB][NT][2]) {
             const int s = unit % STAGES;
-            if (!mbar_wait(&full[s], (unit / STAGES) & 1)) timed_out = true;
+            if (!timed_out && !mbar_wait(&full[s], (unit / STAGES) & 1)) timed_out = true;  // (once one has run out no other is begun)
             const uint32_t base = smem_u32(ring + s * STAGE_BYTES);
 #pragma unroll
             for (int kb = 0; kb < KB; ++kb) {

@@ -77,3 +77,8 @@ def test_a_pair_takes_and_gives_back_its_tensor_memory_when_nothing_else_does():
     assert order == sorted(order)
     behind = text[order[-1]:]
     assert "cluster_sync_all();" in behind[: behind.index("\n}\n")]
+
+
+def test_the_streaming_product_begins_no_wait_behind_one_that_ran_out():
+    waits = [line.strip() for line in SOURCES["gemm_stream.cu"].splitlines() if "mbar_wait(&" in line]
+    assert len(waits) == 3 and all("!timed_out && !mbar_wait(" in line or line.endswith("break;") for line in waits), waits
