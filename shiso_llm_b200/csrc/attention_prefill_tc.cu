@@ -1,11 +1,11 @@
 // Paged attention for long prompt portions on the tensor-memory path (tcgen05), bfloat16,
 // head size 64.
 //
-// One CTA owns 128 rows (token, query head) of one sequence - 128 consecutive tokens of one query head, or, in steps with
-// decoding requests beside a portion, the query heads of one key head, which share its keys and values, for 128 / group consecutive
-// tokens - and walks the key tiles of 64 positions these can see.  (With 128 tokens of one query head a decoding request
-// is a CTA with one row of work per query head: 32 of them beside a portion of 1,024 rows were 1,024 of 1,280
-// CTAs.)  Per tile:
+// One CTA owns 128 rows (token, query head): the query heads of one key head - they share its keys and
+// values - for 128 / group consecutive tokens of one sequence, and walks the key tiles of 64 positions
+// these can see.  (With 128 tokens of one query head instead, a decoding request in a mixed step was a CTA
+// with one row of work per query head: 32 of them beside a portion of 1,024 rows were 1,024 of 1,280 CTAs;
+// and fewer tokens in a tile leave less of the tiles on the diagonal masked.)  Per tile:
 //   S = Q K^T      tcgen05.mma (M 128, N 64, K 64), Q and the key tile in shared memory (K-major,
 //                  128-byte swizzle), S in tensor memory: 128 lanes x 64 float columns, in one of
 //                  two buffers, so that the scores of the tile after next are computed while
@@ -68,7 +68,7 @@ struct TcArgs {
     long long out_ld;
     int* status;
     int width, num_seqs, heads, kv_heads, page_size, window;
-    int pack;                // query heads of a tile: the heads of a key head, or 1
+    int pack;                // query heads of a tile: the heads of a key head (or 1 where a tile would have one token)
     int keep_first;          // with a window: the first positions of a sequence stay visible to every later row
     int cache_rows;          // pages * page size: a row coordinate from here on reads zeros
     float scale_log2;        // scale * log2(e)
@@ -464,20 +464,19 @@ static bool query_map(const void* ptr, int rows, int heads, long long ld, int pa
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// Query heads a tile holds of each token: one, or all that share a key head.  All of them where a step holds decoding requests
-// beside a portion, a sequence for every 128 rows, and a tile then has at least two tokens.  Microseconds with one head and with all,
-// 1,024 rows at 2,048 beside requests of 300 to 700 keys, 32 heads on 8: 32 requests 96 and 59, 15 requests 64 and 50, eight 53 and 50, four and
-// none 49 and 49; 40 heads on one, 32 requests 116 and 82, eight 78 and 77; 63 heads 180 and 93, 97 and 86.  With more than 64 heads a
-// token has tiles of its own, each of which reads all its keys: 72 heads beside 15 requests 134 and 165, 96 heads beside eight 147 and 164.
-// (A prompt alone gains little, 2,048 rows of 32 heads on 8 42 and 40, and keeps one head a tile.)  No bit depends on it.
-static int tile_pack(int heads, int kv_heads, int tokens, int num_seqs) {
+// Query heads a tile holds of each token: all that share a key head, where a tile then has two tokens or more.  Microseconds with one
+// head and with all, 1,024 rows at 2,048 beside requests of 300 to 700 keys, 32 heads on 8: 32 requests 96 and 59, 15 requests 64 and 50,
+// eight 53 and 50, four and none 49 and 49; 2,048 rows alone 42 and 40; 40 heads on one, 32 requests 116 and 82, eight 78 and 77; 63 heads
+// 180 and 93, 97 and 86.  With more than 64 heads a token has tiles of its own, each of which reads all its keys: 72 heads beside 15
+// requests 134 and 165, 96 heads beside eight 147 and 164.  No bit depends on it.
+static int tile_pack(int heads, int kv_heads) {
     const int group = heads / kv_heads;
-    return group <= BQ / 2 && (long long)num_seqs * BQ >= tokens ? group : 1;
+    return group <= BQ / 2 ? group : 1;
 }
 
 // Tokens of a tile: what `max_tiles` of the entry points below counts.
-SHISO_API int shiso_prefill_attention_tc_tile(int heads, int kv_heads, int tokens, int num_seqs) {
-    return kv_heads > 0 && heads % kv_heads == 0 && heads > 0 ? BQ / tile_pack(heads, kv_heads, tokens, num_seqs) : BQ;
+SHISO_API int shiso_prefill_attention_tc_tile(int heads, int kv_heads) {
+    return kv_heads > 0 && heads % kv_heads == 0 && heads > 0 ? BQ / tile_pack(heads, kv_heads) : BQ;
 }
 
 // q [T, heads * 64] bf16 with rows q_ld elements apart, caches [pages, page_size, kv_heads, 64] bf16,
@@ -492,7 +491,7 @@ static int launch_flash_tc(const void* q, long long q_ld, const void* k_cache, c
     if (keep_first < 0) return SHISO_ERR_SHAPE;
     if (kv_heads <= 0 || heads % kv_heads) return SHISO_ERR_SHAPE;
     if (!shiso_prefill_attention_tc_supported(HEAD, page_size)) return SHISO_ERR_UNSUPPORTED;
-    const int pack = tile_pack(heads, kv_heads, tokens, num_seqs);
+    const int pack = tile_pack(heads, kv_heads);
     if ((long long)max_tiles * (heads / pack) > 0x7fffffffLL) return SHISO_ERR_UNSUPPORTED;
     if (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)out) & 15) return SHISO_ERR_ALIGN;
     const long long cache_rows = num_pages * page_size;

@@ -1012,7 +1012,7 @@ def paged_attention(q, heads, kv_heads, head_dim, k_cache, v_cache, block_table,
         and lib.shiso_prefill_attention_tc_supported(head_dim, page_size)
     ):
         # long portions: products in tensor memory, 128 rows (token, query head of a key head) per CTA
-        tiles = _portion_tiles(step, tokens, lib.shiso_prefill_attention_tc_tile(heads, kv_heads, tokens, step.num_seqs))
+        tiles = _portion_tiles(step, tokens, lib.shiso_prefill_attention_tc_tile(heads, kv_heads))
         status = lib.shiso_prefill_attention_tc(
             _ptr(q), _ptr(k_cache), _ptr(v_cache), _ptr(block_table), block_table.shape[1], _ptr(step.q_start),
             _ptr(step.start_pos), _ptr(out), tokens, step.num_seqs, tiles, heads, kv_heads, page_size,
@@ -1352,7 +1352,7 @@ def pooled_window_attention(q, heads, k_cache, v_cache, block_table, pooled_k, p
     ):
         # long portions: the window's tokens by the tensor-memory kernel, which leaves each row's
         # normalised result and the logarithm of its softmax sum; the pooled blocks are folded in after
-        tiles = _portion_tiles(step, tokens, lib.shiso_prefill_attention_tc_tile(heads, kv_heads, tokens, step.num_seqs))
+        tiles = _portion_tiles(step, tokens, lib.shiso_prefill_attention_tc_tile(heads, kv_heads))
         seen = torch.empty((tokens, heads), dtype=torch.float32, device=q.device)
         status = lib.shiso_prefill_attention_tc_open(
             q.data_ptr(), q_ld, _ptr(k_cache), _ptr(v_cache), _ptr(block_table), block_table.shape[1], _ptr(step.q_start),
@@ -1543,7 +1543,7 @@ def masked_attention(q, heads, k_cache, v_cache, block_table, page_size, scale, 
         and getattr(step, "max_q_len", tokens) >= TC_ATTENTION_MIN_PORTION
         and lib.shiso_prefill_attention_tc_supported(dim, page_size)
     ):
-        tiles = _portion_tiles(step, tokens, lib.shiso_prefill_attention_tc_tile(heads, kv_heads, tokens, step.num_seqs))
+        tiles = _portion_tiles(step, tokens, lib.shiso_prefill_attention_tc_tile(heads, kv_heads))
         status = lib.shiso_prefill_attention_tc_kept(
             q.data_ptr(), q_ld, _ptr(k_cache), _ptr(v_cache), _ptr(block_table), block_table.shape[1], _ptr(step.q_start),
             _ptr(step.start_pos), _ptr(out), heads * vdim, tokens, step.num_seqs, tiles, heads, kv_heads, page_size,
