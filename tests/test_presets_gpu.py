@@ -20,20 +20,34 @@ pytestmark = pytest.mark.gpu
 LIMIT_S = 30.0  # a pass takes milliseconds
 
 
-def settle(what):
-    event, began = torch.cuda.Event(), time.monotonic()
-    event.record()
+def poll(event, what):
+    began = time.monotonic()
     while not event.query():
         assert time.monotonic() - began < LIMIT_S, f"{what}: the device did not come to the end of it"
-        time.sleep(0.001)
+        time.sleep(0.0002)
 
 
-@pytest.mark.parametrize("preset,dtype,layers,tokens", [
-    ("lfm2-1.2b", "bfloat16", 0, 700), ("lfm2-350m", "float32", 0, 300), ("volalorn-1b", "bfloat16", 6, 1501), ("filulix-1b", "bfloat16", 6, 1300),
-    ("zetavik-1b", "bfloat16", 6, 600), ("povilorn-350m", "bfloat16", 9, 1100), ("nodepel-350m", "bfloat16", 8, 500), ("raketar-350m", "bfloat16", 8, 500),
-    ("lfm2-350m", "float32", 0, 24), ("volalorn-350m", "bfloat16", 16, 700),
-])
-def test_prompts_of_presets_one_behind_the_other(preset, dtype, layers, tokens):
+class Queue:
+    """At most one step beside the one that runs: a step that stands is met here, with a limit, and not inside the engine."""
+
+    def __init__(self, what):
+        self.what, self.events = what, []
+
+    def put(self, step):
+        if len(self.events) == 2:
+            poll(self.events.pop(0), self.what)
+        out = step()
+        event = torch.cuda.Event()
+        event.record()
+        self.events.append(event)
+        return out
+
+    def empty(self):
+        while self.events:
+            poll(self.events.pop(0), self.what)
+
+
+def engine_of(preset, dtype, layers, rows, seqs):
     from shiso_llm_b200.kernels import ops
 
     with open(preset_path(preset)) as f:
@@ -44,27 +58,58 @@ def test_prompts_of_presets_one_behind_the_other(preset, dtype, layers, tokens):
     device = torch.device("cuda:0")
     model = Model(plan, BuildEnv(dtype=getattr(torch, dtype), device=device, ops=ops))
     weights = random_device_tensors(model.tensor_specs(), 1, getattr(torch, dtype), device)
-    engine = Engine.from_plan(plan, weights, EngineOptions(dtype=dtype, ctx=2048, page_size=16, kv_cache_tokens=6144, max_num_seqs=8,
-                                                           max_num_batched_tokens=tokens + 64))
+    return plan, Engine.from_plan(plan, weights, EngineOptions(dtype=dtype, ctx=2048, page_size=16, kv_cache_tokens=6144, max_num_seqs=seqs,
+                                                               max_num_batched_tokens=rows))
+
+
+@pytest.mark.parametrize("preset,dtype,layers,tokens", [
+    ("lfm2-1.2b", "bfloat16", 0, 700), ("lfm2-350m", "float32", 0, 300), ("volalorn-1b", "bfloat16", 6, 1501), ("filulix-1b", "bfloat16", 6, 1300),
+    ("zetavik-1b", "bfloat16", 6, 600), ("povilorn-350m", "bfloat16", 9, 1100), ("nodepel-350m", "bfloat16", 8, 500), ("raketar-350m", "bfloat16", 8, 500),
+    ("lfm2-350m", "float32", 0, 24), ("volalorn-350m", "bfloat16", 16, 700),
+])
+def test_prompts_of_presets_one_behind_the_other(preset, dtype, layers, tokens):
+    plan, engine = engine_of(preset, dtype, layers, tokens + 64, 8)
     rng = np.random.RandomState(3)
     prompt = rng.randint(0, plan.vocab_size, tokens).tolist()
     running = [rng.randint(0, plan.vocab_size, 120).tolist() for _ in range(6)]
+    queue = Queue(preset)
 
     def read(turn):
-        logits = engine.step([StepEntry(("p", turn), prompt, [tokens - 1])])
+        logits = queue.put(lambda: engine.step([StepEntry(("p", turn), prompt, [tokens - 1])]))
         engine.finish(("p", turn))
         return logits
 
     first = [read(i).clone() for i in range(3)][-1]  # kernel by kernel, captured, replayed
     for turn in range(3, 63):
         last = read(turn)
-    settle(f"{preset}: 60 prompts")
+    queue.empty()
     assert torch.isfinite(first).all() and torch.equal(first, last)
     for i, t in enumerate(running):
-        engine.step([StepEntry(("r", i), t[:60], [])])
+        queue.put(lambda: engine.step([StepEntry(("r", i), t[:60], [])]))
     for at in range(60, 90):  # a portion beside requests that decode, in the same shape again and again
-        logits = engine.step([StepEntry(("r", i), [t[at]], [0]) for i, t in enumerate(running)] + [StepEntry(("p", at), prompt[: tokens // 2], [tokens // 2 - 1])])
+        entries = [StepEntry(("r", i), [t[at]], [0]) for i, t in enumerate(running)] + [StepEntry(("p", at), prompt[: tokens // 2], [tokens // 2 - 1])]
+        logits = queue.put(lambda: engine.step(entries))
         engine.finish(("p", at))
-    settle(f"{preset}: 30 portions beside decoding requests")
+    queue.empty()
     assert torch.isfinite(logits).all()
-    ops.check_kernel_status()
+    engine.env.ops.check_kernel_status()
+
+
+@pytest.mark.parametrize("preset", ["volalorn-1b", "povilorn-350m", "lfm2-1.2b"])
+def test_a_step_of_eight_prompts_again_and_again(preset):
+    """Eight ragged prompts, padded to 1,984 rows in sixteen sequences: products on pairs of SMs start under the tails of attention with many short
+    tiles.  (With tensor memory taken there a replay stood for good, volalorn-1b's within 7 to some 600.)"""
+    plan, engine = engine_of(preset, "bfloat16", 0, 2100, 8)
+    rng = np.random.RandomState(4)
+    prompts = [rng.randint(0, plan.vocab_size, n).tolist() for n in np.linspace(118, 364, 8).astype(int)]
+    queue = Queue(preset)
+    first = None
+    for turn in range(400):
+        logits = queue.put(lambda: engine.step([StepEntry((turn, i), t, [len(t) - 1]) for i, t in enumerate(prompts)]))
+        for i in range(8):
+            engine.finish((turn, i))
+        if turn == 2:
+            first = logits.clone()
+    queue.empty()
+    assert torch.isfinite(logits).all() and torch.equal(first, logits)
+    engine.env.ops.check_kernel_status()
